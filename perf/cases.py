@@ -147,13 +147,23 @@ def prepare(case, seed):
     if _stream is None:
         _stream = torch.cuda.Stream()  # a program's own stream: the default one cannot be captured
     hom.set_stream(_stream.cuda_stream)
-    gen = torch.Generator(device="cuda")
-    gen.manual_seed(seed)
-    rng = np.random.default_rng(seed)
+    gen, rng = _sources(seed)
     state = {"case": case, "hom": hom, "call": getattr(sys.modules[__name__], "_run_" + case["kind"])}
     getattr(sys.modules[__name__], "_prepare_" + case["kind"])(case, state, gen, rng)
     _stream.wait_stream(torch.cuda.current_stream())
     return state
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, in 64 bits with plain torch (no rounding in between)."""
+    with torch.no_grad():
+        return getattr(sys.modules[__name__], "_exact_" + case["kind"])(case, *_sources(seed))
+
+
+def _sources(seed):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    return gen, np.random.default_rng(seed)
 
 
 def run(state):
@@ -175,17 +185,29 @@ def _memref(tensor):
 
 # ------------------------------------------------------------------------------- encoder
 
+def _encoder_inputs(case, gen, rng):
+    """Weights in call order, then token ids and mask on the host."""
+    m = _MODELS[case["model"]]
+    batch, seq, h, f = case["batch"], case["seq"], m["hidden"], m["ffn"]
+    shapes = {"word_emb": (1, _VOCAB, h), "pos_emb": (1, seq, h), "type_emb": (1, 2, h)}
+    for i in range(m["layers"]):
+        for name, (k, n) in {"wqkv": (h, 3 * h), "wo": (h, h), "w1": (h, f), "w2": (f, h)}.items():
+            shapes[f"{name}_{i}"] = (1, n, k) if case["nk"] else (1, k, n)
+    weights = {name: _normal(gen, shape, 0.02) for name, shape in shapes.items()}
+    ids = rng.integers(1000, _VOCAB, (batch, seq)).astype(np.int64)
+    lengths = rng.integers(case["shortest"], seq + 1, batch)
+    mask = (np.arange(seq)[None, :] < lengths[:, None]).astype(np.int64)
+    return weights, ids, mask
+
+
 def _prepare_encoder(case, state, gen, rng):
     mod = _program_module()
     cfg = mod.BertConfig(vocab=_VOCAB, type_vocab=2, eps=_EPS, **_MODELS[case["model"]])
     batch, seq = case["batch"], case["seq"]
-    weights = {name: _normal(gen, cfg.weight_shape(name, seq, case["nk"]), 0.02) for name in cfg.weight_names()}
+    weights, ids, mask = _encoder_inputs(case, gen, rng)
     program = mod.BertProgram(cfg, batch, seq, weights_nk=case["nk"])
     program.set_weights(weights)
-    ids = rng.integers(1000, _VOCAB, (batch, seq))
-    lengths = rng.integers(case["shortest"], seq + 1, batch)
-    mask = (np.arange(seq)[None, :] < lengths[:, None]).astype(np.int64)
-    inputs = [torch.from_numpy(x.astype(np.int64)) for x in (ids, mask, np.zeros_like(ids))]
+    inputs = [torch.from_numpy(x) for x in (ids, mask, np.zeros_like(ids))]
     if case["mode"] == "host":
         state["inputs"] = [x.pin_memory() for x in inputs]
         state["out"] = torch.empty((batch, seq, cfg.hidden), dtype=torch.float16).pin_memory()
@@ -203,14 +225,58 @@ def _run_encoder(hom, state):
     return torch.as_tensor(_DeviceResult(program, memref), device="cuda")
 
 
+def _exact_encoder(case, gen, rng):
+    weights, ids, mask = _encoder_inputs(case, gen, rng)
+    m = _MODELS[case["model"]]
+
+    def matrix(name):
+        w = weights[name][0].double()
+        return w.t() if case["nk"] else w
+
+    valid = torch.from_numpy(mask.astype(bool)).cuda()
+    ids = torch.from_numpy(ids).cuda()
+    x = weights["word_emb"][0][ids].double() + weights["type_emb"][0][0].double() + weights["pos_emb"][0].double()
+    x = _layernorm64(x, _EPS)
+    for i in range(m["layers"]):
+        qkv = x @ matrix(f"wqkv_{i}")
+        x = _layernorm64(_attention64(qkv, valid, m["heads"]) @ matrix(f"wo_{i}") + x, _EPS)
+        del qkv
+        hidden = x @ matrix(f"w1_{i}")
+        x = _layernorm64(torch.nn.functional.gelu(hidden) @ matrix(f"w2_{i}") + x, _EPS)
+    return x
+
+
+def _layernorm64(x, eps):
+    return torch.nn.functional.layer_norm(x, x.shape[-1:], eps=eps)
+
+
+def _attention64(qkv, valid, heads):
+    """Keys of padding are left out, query rows of padding are zero; a few sequences at a time."""
+    batch, seq, _ = qkv.shape
+    out = torch.zeros((batch, seq, heads * 64), dtype=torch.float64, device=qkv.device)
+    step = max(1, (1 << 28) // (heads * seq * seq))
+    for lo in range(0, batch, step):
+        part = qkv[lo:lo + step].reshape(-1, seq, 3, heads, 64)
+        q, k, v = (part[:, :, i].transpose(1, 2) for i in range(3))
+        here = valid[lo:lo + step]
+        scores = (q @ k.transpose(-1, -2) * 0.125).masked_fill(~here[:, None, None, :], float("-inf"))
+        rows = (torch.softmax(scores, -1) @ v).transpose(1, 2).reshape(-1, seq, heads * 64)
+        out[lo:lo + step] = rows * here[:, :, None]
+    return out
+
+
 # ---------------------------------------------------------------------- single entry points
 
-def _prepare_gemm_gelu(case, state, gen, rng):
+def _gemm_gelu_inputs(case, gen, rng):
     m, n, k = case["m"], case["n"], case["k"]
-    state["weight"] = _Weight(state["hom"], _normal(gen, (1, k, n), 0.02))
-    state["out"] = torch.empty((1, m, n), dtype=torch.float16, device="cuda")
-    state["args"] = [_memref(t) for t in (_uniform(gen, (1, m, k)), state["weight"].tensor, _uniform(gen, (1, 1, n)),
-                                          state["out"])]
+    return _normal(gen, (1, k, n), 0.02), _uniform(gen, (1, m, k)), _uniform(gen, (1, 1, n))
+
+
+def _prepare_gemm_gelu(case, state, gen, rng):
+    weight, x, bias = _gemm_gelu_inputs(case, gen, rng)
+    state["weight"] = _Weight(state["hom"], weight)
+    state["out"] = torch.empty((1, case["m"], case["n"]), dtype=torch.float16, device="cuda")
+    state["args"] = [_memref(t) for t in (x, weight, bias, state["out"])]
 
 
 def _run_gemm_gelu(hom, state):
@@ -218,12 +284,21 @@ def _run_gemm_gelu(hom, state):
     return state["out"]
 
 
-def _prepare_layernorm(case, state, gen, rng):
+def _exact_gemm_gelu(case, gen, rng):
+    weight, x, bias = (t.double() for t in _gemm_gelu_inputs(case, gen, rng))
+    return torch.nn.functional.gelu(x @ weight + bias)
+
+
+def _layernorm_inputs(case, gen, rng):
     rows, hidden = case["rows"], case["hidden"]
-    state["out"] = torch.empty((1, rows, hidden), dtype=torch.float16, device="cuda")
-    state["args"] = [_memref(t) for t in (_normal(gen, (1, rows, hidden)), _normal(gen, (1, rows, hidden)),
-                                          _normal(gen, (hidden,), 0.1, 1.0), _normal(gen, (hidden,), 0.1),
-                                          state["out"])]
+    return (_normal(gen, (1, rows, hidden)), _normal(gen, (1, rows, hidden)), _normal(gen, (hidden,), 0.1, 1.0),
+            _normal(gen, (hidden,), 0.1))
+
+
+def _prepare_layernorm(case, state, gen, rng):
+    inputs = _layernorm_inputs(case, gen, rng)
+    state["out"] = torch.empty_like(inputs[0])
+    state["args"] = [_memref(t) for t in (*inputs, state["out"])]
 
 
 def _run_layernorm(hom, state):
@@ -231,12 +306,23 @@ def _run_layernorm(hom, state):
     return state["out"]
 
 
-def _prepare_attention(case, state, gen, rng):
+def _exact_layernorm(case, gen, rng):
+    x, residual, gamma, beta = (t.double() for t in _layernorm_inputs(case, gen, rng))
+    return torch.nn.functional.layer_norm(x + residual, x.shape[-1:], gamma, beta, eps=_EPS)
+
+
+def _attention_inputs(case, gen, rng):
     batch, seq, heads = case["batch"], case["seq"], case["heads"]
     lengths = rng.integers(case["shortest"], seq + 1, batch)
+    return lengths, _normal(gen, (batch, seq, 3 * heads * 64))
+
+
+def _prepare_attention(case, state, gen, rng):
+    lengths, qkv = _attention_inputs(case, gen, rng)
+    batch, seq, heads = case["batch"], case["seq"], case["heads"]
     cu = torch.from_numpy(np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)).cuda()
     state["out"] = torch.empty((batch, seq, heads * 64), dtype=torch.float16, device="cuda")
-    state["args"] = [_memref(t) for t in (_normal(gen, (batch, seq, 3 * heads * 64)), cu, state["out"])]
+    state["args"] = [_memref(t) for t in (qkv, cu, state["out"])]
     state["heads"] = heads
 
 
@@ -245,18 +331,28 @@ def _run_attention(hom, state):
     return state["out"]
 
 
-def _prepare_ln_pair(case, state, gen, rng):
+def _exact_attention(case, gen, rng):
+    lengths, qkv = _attention_inputs(case, gen, rng)
+    valid = torch.from_numpy(np.arange(case["seq"])[None, :] < lengths[:, None]).cuda()
+    return _attention64(qkv.double(), valid, case["heads"])
+
+
+def _ln_pair_inputs(case, gen, rng):
     m, k, n, n2 = case["m"], case["k"], case["n"], case["n2"]
+    return (_normal(gen, (1, k, n), 0.02), _normal(gen, (1, n, n2), 0.02), _normal(gen, (1, m, n)),
+            _normal(gen, (1, 1, n2), 0.1), _normal(gen, (1, m, k)))
+
+
+def _prepare_ln_pair(case, state, gen, rng):
+    m, n, n2 = case["m"], case["n"], case["n2"]
     half = dict(dtype=torch.float16, device="cuda")
-    state["weights"] = [_Weight(state["hom"], _normal(gen, (1, k, n), 0.02)),
-                        _Weight(state["hom"], _normal(gen, (1, n, n2), 0.02))]
-    residual, bias = _normal(gen, (1, m, n)), _normal(gen, (1, 1, n2), 0.1)
+    first, second, residual, bias, x = _ln_pair_inputs(case, gen, rng)
+    state["weights"] = [_Weight(state["hom"], first), _Weight(state["hom"], second)]
     state["outs"] = [torch.empty((1, m, n), **half), torch.empty((m,), **half), torch.empty((m,), **half),
                      torch.empty((1, m, n2), **half)]
     hidden, var, mean, out = (_memref(t) for t in state["outs"])
-    w1, w2 = (_memref(w.tensor) for w in state["weights"])
-    state["first"] = [_memref(_normal(gen, (1, m, k))), w1, _memref(residual), hidden, var, mean]
-    state["second"] = [hidden, w2, _memref(bias), out, var, mean]
+    state["first"] = [_memref(x), _memref(first), _memref(residual), hidden, var, mean]
+    state["second"] = [hidden, _memref(second), _memref(bias), out, var, mean]
 
 
 def _run_ln_pair(hom, state):
@@ -265,17 +361,35 @@ def _run_ln_pair(hom, state):
     return state["outs"]
 
 
-def _prepare_vocab(case, state, gen, rng):
+def _exact_ln_pair(case, gen, rng):
+    """The statistics travel as 1/std and -mean/std."""
+    first, second, residual, bias, x = (t.double() for t in _ln_pair_inputs(case, gen, rng))
+    hidden = x @ first + residual
+    mean = hidden.mean(-1, keepdim=True)
+    rstd = ((hidden - mean).square().mean(-1, keepdim=True) + 1e-5).rsqrt()
+    return [hidden, rstd.reshape(-1), (-mean * rstd).reshape(-1), (hidden - mean) * rstd @ second + bias]
+
+
+def _vocab_inputs(case, gen, rng):
     m, n, k = case["m"], case["n"], case["k"]
-    state["weight"] = _Weight(state["hom"], _normal(gen, (1, k, n), 0.02))
-    state["out"] = torch.empty((1, m, n), dtype=torch.float16, device="cuda")
-    state["args"] = [_memref(t) for t in (_normal(gen, (1, m, k)), state["weight"].tensor,
-                                          _normal(gen, (1, 1, n), 0.02), state["out"])]
+    return _normal(gen, (1, k, n), 0.02), _normal(gen, (1, m, k)), _normal(gen, (1, 1, n), 0.02)
+
+
+def _prepare_vocab(case, state, gen, rng):
+    weight, x, bias = _vocab_inputs(case, gen, rng)
+    state["weight"] = _Weight(state["hom"], weight)
+    state["out"] = torch.empty((1, case["m"], case["n"]), dtype=torch.float16, device="cuda")
+    state["args"] = [_memref(t) for t in (x, weight, bias, state["out"])]
 
 
 def _run_vocab(hom, state):
     hom.cutlassGemmF16(*state["args"], activation=0, alpha=1.0, beta=1.0)
     return state["out"]
+
+
+def _exact_vocab(case, gen, rng):
+    weight, x, bias = (t.double() for t in _vocab_inputs(case, gen, rng))
+    return x @ weight + bias
 
 
 # ------------------------------------------------------------------------ work and tolerance
