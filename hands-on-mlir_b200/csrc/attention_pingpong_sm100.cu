@@ -158,139 +158,144 @@ attention_f16_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const P
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    const bool leader = elect_one();
-    uint32_t q_uses[2] = {0, 0};  // completed loads into each Q buffer
-    uint32_t kv_uses = 0;         // K / V tiles loaded so far (stage = kv_uses % kKvStages)
-    bool ok = true;
-    for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
-      const Item it = decode_item(p, item);
-      if (!it.act[0]) continue;  // tile B cannot be active without tile A
-      const int row_base = it.batch * p.seq;
-      for (int t = 0; t < 2 && ok; ++t) {
-        if (!it.act[t]) continue;
-        // the buffer is free once every S MMA of the item that used it last has completed
-        const int b = q_uses[t] & 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait(q_empty(t, b), ((q_uses[t] >> 1) & 1u) ^ 1u, abort_flag, p.status,
-                                               kDevWaitTimeoutAttention));
-        if (!ok) break;
-        if (leader) {
+    // One elected lane runs the whole loop: see the MMA issuer.
+    if (elect_one()) {
+      uint32_t q_uses[2] = {0, 0};  // completed loads into each Q buffer
+      uint32_t kv_uses = 0;         // K / V tiles loaded so far (stage = kv_uses % kKvStages)
+      bool ok = true;
+      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
+        const Item it = decode_item(p, item);
+        if (!it.act[0]) continue;  // tile B cannot be active without tile A
+        const int row_base = it.batch * p.seq;
+        for (int t = 0; t < 2 && ok; ++t) {
+          if (!it.act[t]) continue;
+          // the buffer is free once every S MMA of the item that used it last has completed
+          const int b = q_uses[t] & 1u;
+          ok = mbar_wait(q_empty(t, b), ((q_uses[t] >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitTimeoutAttention);
+          if (!ok) break;
           mbar_arrive_expect_tx(q_full(t, b), kTileBytes);
           tma_load_2d(smem_base + kOffQ + (2 * t + b) * kTileBytes, &tmQKV, q_full(t, b), it.head * kHeadDim,
                       row_base + it.q0 + t * kTile);
+          ++q_uses[t];
         }
-        ++q_uses[t];
-      }
-      for (int j = 0; j < it.n_kv && ok; ++j) {
-        const int s = kv_uses % kKvStages;
-        const uint32_t ph = (kv_uses / kKvStages) & 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait(k_empty(s), ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutAttention));
-        if (!ok) break;
-        if (leader) {
+        for (int j = 0; j < it.n_kv && ok; ++j) {
+          const int s = kv_uses % kKvStages;
+          const uint32_t ph = (kv_uses / kKvStages) & 1u;
+          ok = mbar_wait(k_empty(s), ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutAttention);
+          if (!ok) break;
           mbar_arrive_expect_tx(k_full(s), kTileBytes);
           tma_load_2d(smem_base + kOffK + s * kTileBytes, &tmQKV, k_full(s), hidden + it.head * kHeadDim,
                       row_base + j * kTile);
-        }
-        ok = __all_sync(0xffffffffu, mbar_wait(v_empty(s), ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutAttention));
-        if (!ok) break;
-        if (leader) {
+          ok = mbar_wait(v_empty(s), ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutAttention);
+          if (!ok) break;
           mbar_arrive_expect_tx(v_full(s), kTileBytes);
           tma_load_2d(smem_base + kOffV + s * kTileBytes, &tmQKV, v_full(s), 2 * hidden + it.head * kHeadDim,
                       row_base + j * kTile);
+          ++kv_uses;
         }
-        ++kv_uses;
+      }
+      if (!ok) {
+        // Give copies already in flight time to land before shared memory is released.
+        const long long t0 = clock64();
+        while (clock64() - t0 < 4000000LL) {
+        }
       }
     }
-    if (!ok) {
-      // Give copies already in flight time to land before shared memory is released.
-      const long long t0 = clock64();
-      while (clock64() - t0 < 4000000LL) {
-      }
-    }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    // The whole warp runs the loop (addresses and descriptors stay warp-uniform); one elected
-    // lane issues the MMAs and the commits.
-    constexpr uint32_t idesc_s = make_idesc_f16(kTile, kTile, false, false);
-    constexpr uint32_t idesc_o = make_idesc_f16(kTile, kHeadDim, false, true);
-    const bool leader = elect_one();
-    uint32_t q_uses[2] = {0, 0}, kv_uses = 0;
-    uint32_t p_uses[2] = {0, 0}, o_uses[2] = {0, 0};
-    bool ok = true;
-    auto wait = [&](uint32_t bar, uint32_t parity) {
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.status, kDevWaitTimeoutAttention));
-      tc_fence_after_sync();
-      return ok;
-    };
-    auto issue_s = [&](int t, int stage, int q_buf) {
-      const uint32_t q_addr = smem_base + kOffQ + (2 * t + q_buf) * kTileBytes;
-      const uint32_t k_addr = smem_base + kOffK + stage * kTileBytes;
+    // One lane, elected once around the whole loop, so that an MMA costs an issue slot and not a
+    // vote, a re-election and a reconvergence of the warp (about 100 clk each: with twelve MMAs
+    // per query tile and KV step that was most of a step).
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_f16(kTile, kTile, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(kTile, kHeadDim, false, true);
+      uint32_t q_uses[2] = {0, 0}, kv_uses = 0;
+      uint32_t p_uses[2] = {0, 0}, o_uses[2] = {0, 0};
+      bool ok = true;
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        ok = mbar_wait(bar, parity, abort_flag, p.status, kDevWaitTimeoutAttention);
+        tc_fence_after_sync();
+        return ok;
+      };
+      auto issue_s = [&](int t, int stage, int q_buf) {
+        const uint32_t q_addr = smem_base + kOffQ + (2 * t + q_buf) * kTileBytes;
+        const uint32_t k_addr = smem_base + kOffK + stage * kTileBytes;
+        const uint64_t da = make_smem_desc_sw128(q_addr, 16, 1024), db = make_smem_desc_sw128(k_addr, 16, 1024);
 #pragma unroll
-      for (int k = 0; k < kHeadDim / 16; ++k) {
-        const uint64_t da = make_smem_desc_sw128(q_addr + k * 32, 16, 1024);
-        const uint64_t db = make_smem_desc_sw128(k_addr + k * 32, 16, 1024);
-        if (leader) tc_mma_f16_ss(tmem_base + t * kTile, da, db, idesc_s, k != 0 ? 1u : 0u);
-      }
-      if (leader) tc_commit(s_full(t));
-    };
-    for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
-      const Item it = decode_item(p, item);
-      if (!it.act[0]) continue;
-      const int n_act = it.act[1] ? 2 : 1;
-      int qb[2] = {0, 0};
-      for (int t = 0; t < n_act && ok; ++t) {
-        qb[t] = q_uses[t] & 1u;
-        wait(q_full(t, qb[t]), (q_uses[t] >> 1) & 1u);
-        ++q_uses[t];
-      }
-      if (!ok) break;
-      // S of the first KV tile for both query tiles
-      {
-        const int s = kv_uses % kKvStages;
-        if (!wait(k_full(s), (kv_uses / kKvStages) & 1u)) break;
-        for (int t = 0; t < n_act; ++t) issue_s(t, s, qb[t]);
-        if (leader) tc_commit(k_empty(s));
-      }
-      for (int j = 0; j < it.n_kv && ok; ++j) {
-        const int s = (kv_uses + j) % kKvStages;
-        const uint32_t ph = ((kv_uses + j) / kKvStages) & 1u;
-        const int valid = min(kTile, it.len - j * kTile);
-        const int k_steps = (valid + 15) >> 4;  // key groups that hold a valid key
-        const int s_next = (kv_uses + j + 1) % kKvStages;
-        const uint32_t ph_next = ((kv_uses + j + 1) / kKvStages) & 1u;
-        if (!wait(v_full(s), ph)) break;
+        for (int k = 0; k < kHeadDim / 16; ++k)
+          tc_mma_f16_ss(tmem_base + t * kTile, smem_desc_advance(da, k * 32), smem_desc_advance(db, k * 32), idesc_s,
+                        k != 0 ? 1u : 0u);
+        tc_commit(s_full(t));
+      };
+      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
+        const Item it = decode_item(p, item);
+        if (!it.act[0]) continue;
+        const int n_act = it.act[1] ? 2 : 1;
+        int qb[2] = {0, 0};
         for (int t = 0; t < n_act && ok; ++t) {
-          // P_t of this step is in shared memory and S_t has been read
-          if (!wait(p_full(t), p_uses[t] & 1u)) break;
-          ++p_uses[t];
-          // S of the next KV tile first: the tile's threads need it before they need O
-          if (j + 1 < it.n_kv) {
-            if (t == 0 && !wait(k_full(s_next), ph_next)) break;
-            issue_s(t, s_next, qb[t]);
-            if (t == n_act - 1 && leader) tc_commit(k_empty(s_next));
-          }
-          // the O buffer this step writes was last read two steps ago
-          const int ob = o_uses[t] & 1u;
-          if (!wait(o_empty(t, ob), ((o_uses[t] >> 1) & 1u) ^ 1u)) break;
-          ++o_uses[t];
-          const uint32_t p_addr = smem_base + kOffP + t * 2 * kTileBytes;
-          const uint32_t v_addr = smem_base + kOffV + s * kTileBytes;
-          const uint32_t o_tmem = tmem_base + 2 * kTile + (2 * t + ob) * kHeadDim;
-          for (int k = 0; k < k_steps; ++k) {
-            const uint64_t da = make_smem_desc_sw128(p_addr + (k >> 2) * kTileBytes + (k & 3) * 32, 16, 1024);
-            // V tile: 128 kv rows of 128 B; N (= d) contiguous, 16 kv rows = 2048 B.
-            const uint64_t db = make_smem_desc_sw128(v_addr + k * 2048, kTileBytes, 1024);
-            if (leader) tc_mma_f16_ss(o_tmem, da, db, idesc_o, k != 0 ? 1u : 0u);
-          }
-          if (leader) tc_commit(o_full(t, ob));
+          qb[t] = q_uses[t] & 1u;
+          wait(q_full(t, qb[t]), (q_uses[t] >> 1) & 1u);
+          ++q_uses[t];
         }
-        if (ok && leader) tc_commit(v_empty(s));
+        if (!ok) break;
+        // S of the first KV tile for both query tiles
+        {
+          const int s = kv_uses % kKvStages;
+          if (!wait(k_full(s), (kv_uses / kKvStages) & 1u)) break;
+          for (int t = 0; t < n_act; ++t) issue_s(t, s, qb[t]);
+          tc_commit(k_empty(s));
+        }
+        for (int j = 0; j < it.n_kv && ok; ++j) {
+          const int s = (kv_uses + j) % kKvStages;
+          const uint32_t ph = ((kv_uses + j) / kKvStages) & 1u;
+          const int valid = min(kTile, it.len - j * kTile);
+          const int k_steps = (valid + 15) >> 4;  // key groups that hold a valid key
+          const int s_next = (kv_uses + j + 1) % kKvStages;
+          const uint32_t ph_next = ((kv_uses + j + 1) / kKvStages) & 1u;
+          if (!wait(v_full(s), ph)) break;
+          for (int t = 0; t < n_act && ok; ++t) {
+            // P_t of this step is in shared memory and S_t has been read
+            if (!wait(p_full(t), p_uses[t] & 1u)) break;
+            ++p_uses[t];
+            // S of the next KV tile first: the tile's threads need it before they need O
+            if (j + 1 < it.n_kv) {
+              if (t == 0 && !wait(k_full(s_next), ph_next)) break;
+              issue_s(t, s_next, qb[t]);
+              if (t == n_act - 1) tc_commit(k_empty(s_next));
+            }
+            // the O buffer this step writes was last read two steps ago
+            const int ob = o_uses[t] & 1u;
+            if (!wait(o_empty(t, ob), ((o_uses[t] >> 1) & 1u) ^ 1u)) break;
+            ++o_uses[t];
+            const uint32_t p_addr = smem_base + kOffP + t * 2 * kTileBytes;
+            const uint32_t v_addr = smem_base + kOffV + s * kTileBytes;
+            const uint32_t o_tmem = tmem_base + 2 * kTile + (2 * t + ob) * kHeadDim;
+            // V tile: 128 kv rows of 128 B; N (= d) contiguous, 16 kv rows = 2048 B.
+            const uint64_t da = make_smem_desc_sw128(p_addr, 16, 1024);
+            const uint64_t db = make_smem_desc_sw128(v_addr, kTileBytes, 1024);
+            auto step = [&](int k) {
+              tc_mma_f16_ss(o_tmem, smem_desc_advance(da, (k >> 2) * kTileBytes + (k & 3) * 32),
+                            smem_desc_advance(db, k * 2048), idesc_o, k != 0 ? 1u : 0u);
+            };
+            if (k_steps == kTile / 16) {
+#pragma unroll
+              for (int k = 0; k < kTile / 16; ++k) step(k);
+            } else {
+              for (int k = 0; k < k_steps; ++k) step(k);
+            }
+            tc_commit(o_full(t, ob));
+          }
+          if (ok) tc_commit(v_empty(s));
+        }
+        // every S MMA of the item has been issued: the Q buffers are free once they complete
+        if (ok) {
+          for (int t = 0; t < n_act; ++t) tc_commit(q_empty(t, qb[t]));
+        }
+        kv_uses += it.n_kv;
       }
-      // every S MMA of the item has been issued: the Q buffers are free once they complete
-      if (ok && leader) {
-        for (int t = 0; t < n_act; ++t) tc_commit(q_empty(t, qb[t]));
-      }
-      kv_uses += it.n_kv;
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------ softmax, one query row per thread
     const int t = (warp - 2) >> 2;             // which query tile of the pair

@@ -426,10 +426,9 @@ attention_f16_single_tile_kernel(const __grid_constant__ CUtensorMap tmQKV,
   pdl_wait();  // cu_seqlens and the packed QKV come from earlier kernels of the stream
   stamp(1);
   // The tiles do not depend on the valid length: request them before reading it.
-  // Warp 0 runs the copy / MMA issue code as a whole (addresses and descriptors stay
-  // warp-uniform); one elected lane executes the asynchronous instructions.
-  const bool leader = warp == 0 && elect_one();
-  if (leader) {
+  // Copies and MMAs are issued by one elected lane of warp 0, each block of them under one
+  // election (elect.sync names the same lane every time).
+  if (warp == 0 && elect_one()) {
     const int row_base = batch * p.seq;
     mbar_arrive_expect_tx(bar_load, 2 * kTileBytes);
     tma_load_2d(smem_q, &tmQKV, bar_load, head * kHeadDim, row_base);
@@ -449,13 +448,15 @@ attention_f16_single_tile_kernel(const __grid_constant__ CUtensorMap tmQKV,
         stamp(3);
         tc_fence_after_sync();
         constexpr uint32_t idesc_s = make_idesc_f16(kTile, kTile, false, false);
+        if (elect_one()) {
+          const uint64_t da = make_smem_desc_sw128(smem_q, 16, 1024), db = make_smem_desc_sw128(smem_k, 16, 1024);
 #pragma unroll
-        for (int k = 0; k < kHeadDim / 16; ++k) {
-          const uint64_t da = make_smem_desc_sw128(smem_q + k * 32, 16, 1024);
-          const uint64_t db = make_smem_desc_sw128(smem_k + k * 32, 16, 1024);
-          if (leader) tc_mma_f16_ss(tmem_acc, da, db, idesc_s, k != 0 ? 1u : 0u);
+          for (int k = 0; k < kHeadDim / 16; ++k)
+            tc_mma_f16_ss(tmem_acc, smem_desc_advance(da, k * 32), smem_desc_advance(db, k * 32), idesc_s,
+                          k != 0 ? 1u : 0u);
+          tc_commit(bar_s);
         }
-        if (leader) tc_commit(bar_s);
+        __syncwarp();
       }
     }
     ok = mbar_wait(bar_s, 0, abort_flag, p.status, kDevWaitTimeoutAttention);
@@ -545,13 +546,17 @@ attention_f16_single_tile_kernel(const __grid_constant__ CUtensorMap tmQKV,
         tc_fence_after_sync();
         constexpr uint32_t idesc_o = make_idesc_f16(kTile, kHeadDim, false, true);
         const int k_steps = (len + 15) >> 4;  // key groups beyond the last valid key hold no P
-        for (int k = 0; k < k_steps; ++k) {
-          const uint64_t da =
-              make_smem_desc_sw128(smem_p + (k >> 2) * kTileBytes + (k & 3) * 32, 16, 1024);
-          const uint64_t db = make_smem_desc_sw128(smem_v + k * 2048, kTileBytes, 1024);
-          if (leader) tc_mma_f16_ss(tmem_acc, da, db, idesc_o, k != 0 ? 1u : 0u);
+        if (elect_one()) {
+          const uint64_t da = make_smem_desc_sw128(smem_p, 16, 1024);
+          const uint64_t db = make_smem_desc_sw128(smem_v, kTileBytes, 1024);
+#pragma unroll
+          for (int k = 0; k < kTile / 16; ++k)
+            if (k < k_steps)
+              tc_mma_f16_ss(tmem_acc, smem_desc_advance(da, (k >> 2) * kTileBytes + (k & 3) * 32),
+                            smem_desc_advance(db, k * 2048), idesc_o, k != 0 ? 1u : 0u);
+          tc_commit(bar_o);
         }
-        if (leader) tc_commit(bar_o);
+        __syncwarp();
       }
       ok = mbar_wait(bar_o, 0, abort_flag, p.status, kDevWaitTimeoutAttention);
       ok = __syncthreads_and(ok);
@@ -599,7 +604,7 @@ attention_f16_single_tile_kernel(const __grid_constant__ CUtensorMap tmQKV,
     tc_fence_before_sync();
     __syncthreads();
     stamp(8);
-    if (leader) {
+    if (warp == 0 && elect_one()) {
       asm volatile(
           "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
           :

@@ -52,7 +52,6 @@ struct PairParams {
   EpilogueParams ep;
   int K;
   int n_blocks, num_tiles, num_kb;
-  int stages;
   int b_grouped;  // B [K,N] is fetched through the grouped 3-D tensor map (N % 64 == 0)
   int b_early;    // B is a declared constant: request its first tiles before griddepcontrol.wait
   // Split-K: every tile is cut into `split_k` work units (K-block ranges); num_units = num_tiles
@@ -73,7 +72,6 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   using Cfg = PairCfg<BN2>;
   constexpr int STAGES = Cfg::kStages;
   constexpr int HALF = Cfg::kHalfN;
-  const int stages_used = p.stages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t smem_base = (raw_addr + 1023u) & ~1023u;
@@ -136,32 +134,32 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    // Run by the whole warp (coordinates and addresses stay warp-uniform); one elected lane
-    // arms the barriers and issues the copies.
-    {
-      const bool leader = elect_one();
-      int s = 0;
-      uint32_t ph = 0;
+    // One elected lane runs the whole loop (see gemm_sm100.cu).
+    if (elect_one()) {
+      // Copies of both CTAs complete on the even CTA's barriers, which the even CTA's producer
+      // arms for the bytes of both; `bar` is the stage's barrier in the even CTA (cluster address).
+      const uint32_t full_even = map_to_cta(full_bar(0), 0);
+      uint32_t dst = smem_base, slot = 0, ph = 0;
       bool ok = true;
       HOM_DIAG(long long t_wait = 0; const long long t_begin = clock64();)
-      const uint32_t full_even_base = map_to_cta(full_bar(0), 0);
-      auto full_even = [&](int slot) { return full_even_base + 8u * slot; };
-      auto arm = [&](int slot) {
-        // The even CTA's producer arms the barrier for the bytes of both CTAs; the odd CTA's
-        // copies only count their bytes on it.
-        if (rank == 0 && leader) mbar_arrive_expect_tx(full_bar(slot), 2 * Cfg::kStageBytes);
+      auto advance = [&]() {
+        dst += Cfg::kStageBytes;
+        slot += 8;
+        if (slot == 8 * STAGES) {
+          dst = smem_base;
+          slot = 0;
+          ph ^= 1u;
+        }
       };
-      auto load_b = [&](int slot, int kb, int nb0) {
-        const uint32_t b_dst = smem_base + slot * Cfg::kStageBytes + kABytes;
-        if (!leader) return;
+      const bool b_grouped = p.b_grouped != 0;
+      auto load_b = [&](uint32_t b_dst, uint32_t bar, int k, int nb0) {
         if (B_NK) {
-          tma_load_2d_pair(b_dst, &tmB, full_even(slot), kb * BK, nb0);
-        } else if (p.b_grouped) {
-          tma_load_3d_pair(b_dst, &tmB, full_even(slot), 0, kb * BK, nb0 / 64);
+          tma_load_2d_pair(b_dst, &tmB, bar, k, nb0);
+        } else if (b_grouped) {
+          tma_load_3d_pair(b_dst, &tmB, bar, 0, k, nb0 / 64);
         } else {
 #pragma unroll
-          for (int g = 0; g < HALF / 64; ++g)
-            tma_load_2d_pair(b_dst + g * (BK * 128), &tmB, full_even(slot), nb0 + g * 64, kb * BK);
+          for (int g = 0; g < HALF / 64; ++g) tma_load_2d_pair(b_dst + g * (BK * 128), &tmB, bar, nb0 + g * 64, k);
         }
       };
       // When B is a declared constant (weights, which no kernel of the stream writes) the
@@ -172,44 +170,42 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int tile0 = pair / p.split_k, part0 = pair % p.split_k;
         const int nb0 = (tile0 % p.n_blocks) * BN2 + static_cast<int>(rank) * HALF;
         const int kb0 = part0 * p.num_kb / p.split_k, kb1 = (part0 + 1) * p.num_kb / p.split_k;
-        pre = kb1 - kb0 < stages_used ? kb1 - kb0 : stages_used;
+        pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
         for (int i = 0; i < pre; ++i) {
-          arm(i);
-          load_b(i, kb0 + i, nb0);
+          if (rank == 0) mbar_arrive_expect_tx(full_bar(i), 2 * Cfg::kStageBytes);
+          load_b(smem_base + i * Cfg::kStageBytes + kABytes, full_even + 8u * i, (kb0 + i) * BK, nb0);
         }
       }
       // longest entry -> first weight tiles requested (just before the dependency wait), ns
-      HOM_DIAG(if (p.tl && leader) {
+      HOM_DIAG(if (p.tl) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         atomicMax(p.tl + 481, static_cast<long long>(t - g_entry));
       })
       pdl_wait();
-      HOM_DIAG(if (p.tl && leader) timeline_stamp(p.tl, 2);)
+      HOM_DIAG(if (p.tl) timeline_stamp(p.tl, 2);)
       for (int unit = pair; unit < p.num_units && ok; unit += num_pairs) {
         const int tile = unit / p.split_k, part = unit % p.split_k;
         const int m0 = (tile / p.n_blocks) * 256 + static_cast<int>(rank) * 128;
         const int nb0 = (tile % p.n_blocks) * BN2 + static_cast<int>(rank) * HALF;
-        const int kb_begin = part * p.num_kb / p.split_k, kb_end = (part + 1) * p.num_kb / p.split_k;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          const bool b_done = unit == pair && kb - kb_begin < pre;
-          if (!b_done) {
-            HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
-            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status,
-                                                   kDevWaitTimeoutProducer));
-            if (!ok) break;
-            HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
-            arm(s);
-            load_b(s, kb, nb0);
-          }
-          if (leader) tma_load_2d_pair(smem_base + s * Cfg::kStageBytes, &tmA, full_even(s), kb * BK, m0);
-          if (++s == stages_used) {
-            s = 0;
-            ph ^= 1u;
-          }
+        int k = part * p.num_kb / p.split_k * BK;
+        const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
+        for (; pre > 0; --pre, k += BK) {  // (first unit only: the B half is on its way)
+          tma_load_2d_pair(dst, &tmA, full_even + slot, k, m0);
+          advance();
+        }
+        for (; k < k_end; k += BK) {
+          HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
+          ok = mbar_wait(empty_bar(0) + slot, ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutProducer);
+          if (!ok) break;
+          HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
+          if (rank == 0) mbar_arrive_expect_tx(full_bar(0) + slot, 2 * Cfg::kStageBytes);
+          tma_load_2d_pair(dst, &tmA, full_even + slot, k, m0);
+          load_b(dst + kABytes, full_even + slot, k, nb0);
+          advance();
         }
       }
-      HOM_DIAG(if (p.prof && blockIdx.x < 2 && lane == 0) {
+      HOM_DIAG(if (p.prof && blockIdx.x < 2) {
         p.prof[0 + 8 * blockIdx.x] = clock64() - t_begin;
         p.prof[1 + 8 * blockIdx.x] = t_wait;
       })
@@ -220,15 +216,16 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------- MMA issuer (even CTA only)
-    // The whole warp runs the loop so that stage addresses and descriptors stay warp-uniform;
-    // one elected lane issues the MMAs and the commits.
-    if (rank == 0) {
+    // One elected lane runs the whole loop (see gemm_sm100.cu).
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_f16(256, BN2, false, !B_NK);
-      const bool leader = elect_one();
-      int s = 0;
-      uint32_t ph = 0;
+      const uint64_t da0 = make_smem_desc_sw128(smem_base, 16, 1024);
+      const uint64_t db0 = make_smem_desc_sw128(smem_base + kABytes, B_NK ? 16 : BK * 128, 1024);
+      uint64_t da = da0, db = db0;
+      uint32_t bar = full_bar(0), ph = 0;
       bool ok = true;
       int it = 0;
       HOM_DIAG(long long t_full = 0, t_acc = 0; const long long t_begin = clock64();)
@@ -238,50 +235,43 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         HOM_DIAG(const long long ta = p.prof ? clock64() : 0;)
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait(tempty_bar(acc), acc_ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutMma));
+        ok = mbar_wait(tempty_bar(acc), acc_ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutMma);
         if (!ok) break;
         HOM_DIAG(if (p.prof) t_acc += clock64() - ta;)
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN2;
-        bool have = false;  // full[s] already seen complete by the probe of the previous block
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!have) {
-            HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
-            ok = __all_sync(0xffffffffu,
-                            mbar_wait(full_bar(s), ph, abort_flag, p.status, kDevWaitTimeoutMma));
-            if (!ok) break;
-            HOM_DIAG(if (p.prof) t_full += clock64() - tw;)
-          }
-          have = false;
+          HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
+          ok = mbar_wait(bar, ph, abort_flag, p.status, kDevWaitTimeoutMma);
+          if (!ok) break;
+          HOM_DIAG(if (p.prof) t_full += clock64() - tw;)
           tc_fence_after_sync();
-          HOM_DIAG(if (p.tl && it == 0 && kb == 0 && leader) timeline_stamp(p.tl, 6);)
-          const uint32_t a_addr = smem_base + s * Cfg::kStageBytes;
-          const uint32_t b_addr = a_addr + kABytes;
-          const int s_next = s + 1 == stages_used ? 0 : s + 1;
-          const uint32_t ph_next = s_next == 0 ? ph ^ 1u : ph;
+          HOM_DIAG(if (p.tl && it == 0 && kb == 0) timeline_stamp(p.tl, 6);)
+          tc_mma_f16_ss_pair(d_tmem, da, db, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t da = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            const uint64_t db = B_NK ? make_smem_desc_sw128(b_addr + k * 32, 16, 1024)
-                                     : make_smem_desc_sw128(b_addr + k * 2048, BK * 128, 1024);
-            if (leader) tc_mma_f16_ss_pair(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-            // Probe the next stage while the tensor pipe is busy with what was just queued.
-            if (k == 1 && kb + 1 < num_kb)
-              have = __all_sync(0xffffffffu, mbar_test_wait(full_bar(s_next), ph_next));
+          for (int k = 1; k < BK / 16; ++k)
+            tc_mma_f16_ss_pair(d_tmem, smem_desc_advance(da, k * 32), smem_desc_advance(db, B_NK ? k * 32 : k * 2048),
+                               idesc, 1u);
+          tc_commit_pair(bar + 8u * STAGES, 0x3);  // frees the stage in both CTAs
+          da = smem_desc_advance(da, Cfg::kStageBytes);
+          db = smem_desc_advance(db, Cfg::kStageBytes);
+          bar += 8;
+          if (bar == full_bar(STAGES)) {
+            da = da0;
+            db = db0;
+            bar = full_bar(0);
+            ph ^= 1u;
           }
-          if (leader) tc_commit_pair(empty_bar(s), 0x3);  // frees the stage in both CTAs
-          s = s_next;
-          ph = ph_next;
         }
-        if (ok && leader) tc_commit_pair(tfull_bar(acc), 0x3);  // accumulator ready in both CTAs
+        if (ok) tc_commit_pair(tfull_bar(acc), 0x3);  // accumulator ready in both CTAs
       }
-      HOM_DIAG(if (p.prof && blockIdx.x == 0 && lane == 0) {
+      HOM_DIAG(if (p.prof && blockIdx.x == 0) {
         p.prof[2] = clock64() - t_begin;
         p.prof[3] = t_full;
         p.prof[4] = t_acc;
       })
     }
+    __syncwarp();
   } else if (warp >= kControlWarps) {
     // --------------------------------------------------------------- epilogue
     const int quarter = warp & 3;       // tensor-memory lanes [32*quarter, +32)
@@ -492,11 +482,6 @@ bool launch_pair_variant(const Problem &pb, int split_k, cudaStream_t stream) {
   p.n_blocks = static_cast<int>((pb.N + BN2 - 1) / BN2);
   p.num_tiles = m_blocks * p.n_blocks;
   p.num_kb = static_cast<int>((pb.K + BK - 1) / BK);
-  p.stages = Cfg::kStages;
-  HOM_DIAG(if (const char *env = std::getenv("HOM_GEMM_STAGES")) {  // experiment knob
-    const int v = std::atoi(env);
-    if (v >= 1 && v < Cfg::kStages) p.stages = v;
-  })
   p.status = device_status_word();
   HOM_DIAG(p.prof = profile_buffer(); p.tl = launch_timeline_slot();)
   p.split_k = split_k < 1 || has_layernorm_form(pb) ? 1 : split_k > 16 ? 16 : split_k;

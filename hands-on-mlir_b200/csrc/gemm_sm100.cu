@@ -59,7 +59,6 @@ struct Params {
   EpilogueParams ep;
   int K;
   int n_blocks, num_tiles, num_kb;
-  int stages;  // ring slots in use, <= TileCfg::kStages
   int b_grouped;  // B [K,N] is fetched through the grouped 3-D tensor map (N % 64 == 0)
   int b_early;    // B is a declared constant: request its first tiles before griddepcontrol.wait
   // Split-K: every tile is cut into `split_k` work units (K-block ranges); num_units = num_tiles
@@ -89,8 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmD, const Params p) {
   using Cfg = TileCfg<BN>;
-  constexpr int STAGES = Cfg::kStages;  // ring slots laid out in shared memory
-  const int stages_used = p.stages;
+  constexpr int STAGES = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t smem_base = (raw_addr + 1023u) & ~1023u;
@@ -148,25 +146,31 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    // Run by the whole warp (coordinates and addresses stay warp-uniform); one elected lane
-    // arms the barriers and issues the copies.
-    {
-      const bool leader = elect_one();
-      int s = 0;
-      uint32_t ph = 0, armed = 0;
+    // One elected lane runs the whole loop (see the MMA issuer).
+    if (elect_one()) {
+      // The loop below is a chain of dependent instructions of one thread: addresses advance by
+      // additions, everything else is hoisted (40 clk a K block that the tensor pipe would wait).
+      uint32_t dst = smem_base, bar = full_bar(0), ph = 0, armed = 0;
       bool ok = true;
       HOM_DIAG(long long t_wait = 0; const long long t_begin = clock64();)
-      auto load_b = [&](int slot, int kb, int n0) {
-        const uint32_t b_dst = smem_base + slot * Cfg::kStageBytes + kABytes;
-        if (!leader) return;
+      auto advance = [&]() {
+        dst += Cfg::kStageBytes;
+        bar += 8;
+        if (bar == full_bar(STAGES)) {
+          dst = smem_base;
+          bar = full_bar(0);
+          ph ^= 1u;
+        }
+      };
+      const bool b_grouped = p.b_grouped != 0;
+      auto load_b = [&](uint32_t b_dst, uint32_t b_bar, int k, int n0) {
         if (B_NK) {
-          tma_load_2d(b_dst, &tmB, full_bar(slot), kb * BK, n0);
-        } else if (p.b_grouped) {
-          tma_load_3d(b_dst, &tmB, full_bar(slot), 0, kb * BK, n0 / 64);
+          tma_load_2d(b_dst, &tmB, b_bar, k, n0);
+        } else if (b_grouped) {
+          tma_load_3d(b_dst, &tmB, b_bar, 0, k, n0 / 64);
         } else {
 #pragma unroll
-          for (int g = 0; g < BN / 64; ++g)
-            tma_load_2d(b_dst + g * (BK * 128), &tmB, full_bar(slot), n0 + g * 64, kb * BK);
+          for (int g = 0; g < BN / 64; ++g) tma_load_2d(b_dst + g * (BK * 128), &tmB, b_bar, n0 + g * 64, k);
         }
       };
       // When B is a declared constant (weights, which no kernel of the stream writes) the
@@ -177,60 +181,67 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int tile0 = blockIdx.x / p.split_k, part0 = blockIdx.x % p.split_k;
         const int n0 = (tile0 % p.n_blocks) * BN;
         const int kb0 = part0 * p.num_kb / p.split_k, kb1 = (part0 + 1) * p.num_kb / p.split_k;
-        pre = kb1 - kb0 < stages_used ? kb1 - kb0 : stages_used;
+        pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
         for (int i = 0; i < pre; ++i) {
-          if (leader) mbar_arrive_expect_tx(full_bar(i), Cfg::kStageBytes);
-          load_b(i, kb0 + i, n0);
+          mbar_arrive_expect_tx(full_bar(i), Cfg::kStageBytes);
+          load_b(smem_base + i * Cfg::kStageBytes + kABytes, full_bar(i), (kb0 + i) * BK, n0);
         }
       }
       pdl_wait();
-      HOM_DIAG(if (p.tl && leader) timeline_stamp(p.tl, 2);)
+      HOM_DIAG(if (p.tl) timeline_stamp(p.tl, 2);)
       for (int unit = blockIdx.x; unit < p.num_units && ok; unit += gridDim.x) {
         const int tile = unit / p.split_k, part = unit % p.split_k;
         const int m0 = (tile / p.n_blocks) * BM;
         const int n0 = (tile % p.n_blocks) * BN;
-        const int kb_begin = part * p.num_kb / p.split_k, kb_end = (part + 1) * p.num_kb / p.split_k;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          const bool b_done = unit == static_cast<int>(blockIdx.x) && kb - kb_begin < pre;
-          if (!b_done) {
-            HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
-            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status,
-                                                   kDevWaitTimeoutProducer));
-            if (!ok) break;
-            HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
-            if (leader) mbar_arrive_expect_tx(full_bar(s), Cfg::kStageBytes);
-            load_b(s, kb, n0);
-          }
-          if (leader) tma_load_2d(smem_base + s * Cfg::kStageBytes, &tmA, full_bar(s), kb * BK, m0);
+        int k = part * p.num_kb / p.split_k * BK;
+        const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
+        for (; pre > 0; --pre, k += BK) {  // (first unit only: the B half is on its way)
+          tma_load_2d(dst, &tmA, bar, k, m0);
           ++armed;
-          if (++s == stages_used) {
-            s = 0;
-            ph ^= 1u;
-          }
+          advance();
+        }
+        for (; k < k_end; k += BK) {
+          HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
+          ok = mbar_wait(bar + 8u * STAGES, ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutProducer);
+          if (!ok) break;
+          HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
+          mbar_arrive_expect_tx(bar, Cfg::kStageBytes);
+          tma_load_2d(dst, &tmA, bar, k, m0);
+          load_b(dst + kABytes, bar, k, n0);
+          ++armed;
+          advance();
         }
       }
-      HOM_DIAG(if (p.prof && blockIdx.x == 0 && lane == 0) {
+      HOM_DIAG(if (p.prof && blockIdx.x == 0) {
         p.prof[0] = clock64() - t_begin;
         p.prof[1] = t_wait;
       })
       if (!ok) {
         // Let every copy this warp started land before the CTA gives its shared memory back.
-        for (int st = 0; st < stages_used; ++st) {
-          const uint32_t n_st = armed / stages_used + (static_cast<uint32_t>(st) < armed % stages_used ? 1u : 0u);
+        for (int st = 0; st < STAGES; ++st) {
+          const uint32_t n_st = armed / STAGES + (static_cast<uint32_t>(st) < armed % STAGES ? 1u : 0u);
           if (n_st > 0) mbar_wait_drain(full_bar(st), (n_st - 1u) & 1u);
         }
       }
-      if constexpr (LN) cluster_sync_all();  // the epilogue's statistics exchange counts every thread
     }
+    __syncwarp();
+    if constexpr (LN) cluster_sync_all();  // the epilogue's statistics exchange counts every thread
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    // The whole warp runs the loop so that stage addresses and descriptors stay warp-uniform;
-    // one elected lane issues the MMAs and the commits.
-    {
+    // One lane, elected once by elect.sync around the whole loop: the compiler then knows that a
+    // single thread runs it, and a K block costs the tensor pipe's time.  A loop of the whole warp
+    // with only the issue under the election spends 415-435 clk per 64-deep K block on votes,
+    // reconvergence and re-election, whatever the tile's width; this form 267 / 296 / 401 clk at
+    // N = 64 / 128 / 192, where the pipe itself needs 192 / 256 / 384.
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_f16(BM, BN, false, !B_NK);
-      const bool leader = elect_one();
-      int s = 0;
-      uint32_t ph = 0;
+      // A: K-major rows of 128 B; 8-row groups 1024 B apart; 16 K elements = 32 B.
+      // B as [N,K]: same as A.  B as [K,N] (N contiguous): 64-column groups are separate
+      // sub-tiles BK*128 B apart, 8-row K groups 1024 B apart, and 16 K rows = 2048 B.
+      const uint64_t da0 = make_smem_desc_sw128(smem_base, 16, 1024);
+      const uint64_t db0 = make_smem_desc_sw128(smem_base + kABytes, B_NK ? 16 : BK * 128, 1024);
+      uint64_t da = da0, db = db0;
+      uint32_t bar = full_bar(0), ph = 0;
       bool ok = true;
       int it = 0;
       HOM_DIAG(long long t_full = 0, t_acc = 0; const long long t_begin = clock64();)
@@ -240,54 +251,43 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         HOM_DIAG(const long long ta = p.prof ? clock64() : 0;)
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait(tempty_bar(acc), acc_ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutMma));
+        ok = mbar_wait(tempty_bar(acc), acc_ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutMma);
         if (!ok) break;
         HOM_DIAG(if (p.prof) t_acc += clock64() - ta;)
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        bool have = false;  // full[s] already seen complete by the probe of the previous block
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!have) {
-            HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
-            ok = __all_sync(0xffffffffu,
-                            mbar_wait(full_bar(s), ph, abort_flag, p.status, kDevWaitTimeoutMma));
-            if (!ok) break;
-            HOM_DIAG(if (p.prof) t_full += clock64() - tw;)
-          }
-          have = false;
+          HOM_DIAG(const long long tw = p.prof ? clock64() : 0;)
+          ok = mbar_wait(bar, ph, abort_flag, p.status, kDevWaitTimeoutMma);
+          if (!ok) break;
+          HOM_DIAG(if (p.prof) t_full += clock64() - tw;)
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_base + s * Cfg::kStageBytes;
-          const uint32_t b_addr = a_addr + kABytes;
-          const int s_next = s + 1 == stages_used ? 0 : s + 1;
-          const uint32_t ph_next = s_next == 0 ? ph ^ 1u : ph;
+          tc_mma_f16_ss(d_tmem, da, db, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            // A: K-major rows of 128 B; 8-row groups 1024 B apart; 16 K elements = 32 B.
-            const uint64_t da = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            // B as [N,K]: same as A.  B as [K,N] (N contiguous): 64-column groups are
-            // separate sub-tiles BK*128 B apart, 8-row K groups 1024 B apart, and 16 K rows
-            // = 2048 B.
-            const uint64_t db = B_NK ? make_smem_desc_sw128(b_addr + k * 32, 16, 1024)
-                                     : make_smem_desc_sw128(b_addr + k * 2048, BK * 128, 1024);
-            if (leader) tc_mma_f16_ss(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-            // Probe the next stage while the tensor pipe is busy with what was just queued.
-            if (k == 1 && kb + 1 < num_kb)
-              have = __all_sync(0xffffffffu, mbar_test_wait(full_bar(s_next), ph_next));
+          for (int k = 1; k < BK / 16; ++k)
+            tc_mma_f16_ss(d_tmem, smem_desc_advance(da, k * 32), smem_desc_advance(db, B_NK ? k * 32 : k * 2048),
+                          idesc, 1u);
+          tc_commit(bar + 8u * STAGES);  // frees the stage
+          da = smem_desc_advance(da, Cfg::kStageBytes);
+          db = smem_desc_advance(db, Cfg::kStageBytes);
+          bar += 8;
+          if (bar == full_bar(STAGES)) {
+            da = da0;
+            db = db0;
+            bar = full_bar(0);
+            ph ^= 1u;
           }
-          if (leader) tc_commit(empty_bar(s));
-          s = s_next;
-          ph = ph_next;
         }
-        if (ok && leader) tc_commit(tfull_bar(acc));
+        if (ok) tc_commit(tfull_bar(acc));
       }
-      HOM_DIAG(if (p.prof && blockIdx.x == 0 && lane == 0) {
+      HOM_DIAG(if (p.prof && blockIdx.x == 0) {
         p.prof[2] = clock64() - t_begin;
         p.prof[3] = t_full;
         p.prof[4] = t_acc;
       })
-      if constexpr (LN) cluster_sync_all();  // the epilogue's statistics exchange counts every thread
     }
+    __syncwarp();
+    if constexpr (LN) cluster_sync_all();  // the epilogue's statistics exchange counts every thread
   } else {
     // --------------------------------------------------------------- epilogue
     const int quarter = warp & 3;       // TMEM lanes [32*quarter, 32*quarter + 32)
@@ -683,11 +683,6 @@ bool launch_variant(const Problem &pb, int split_k, cudaStream_t stream) {
   p.n_blocks = static_cast<int>((pb.N + BN - 1) / BN);
   p.num_tiles = m_blocks * p.n_blocks;
   p.num_kb = static_cast<int>((pb.K + BK - 1) / BK);
-  p.stages = Cfg::kStages;
-  HOM_DIAG(if (const char *env = std::getenv("HOM_GEMM_STAGES")) {  // experiment knob
-    const int v = std::atoi(env);
-    if (v >= 1 && v < Cfg::kStages) p.stages = v;
-  })
   p.status = device_status_word();
   HOM_DIAG(p.prof = profile_buffer(); p.tl = launch_timeline_slot();)
   p.split_k = has_layernorm_form(pb) ? 1 : clamp_split(split_k, p.num_kb);
@@ -767,7 +762,6 @@ bool launch_ln_variant(const Problem &pb, float eps, cudaStream_t stream) {
   p.n_blocks = static_cast<int>(pb.N / BN);
   p.num_tiles = m_blocks * p.n_blocks;
   p.num_kb = static_cast<int>((pb.K + BK - 1) / BK);
-  p.stages = Cfg::kStages;
   p.status = device_status_word();
   HOM_DIAG(p.prof = nullptr; p.tl = nullptr;)
   p.split_k = 1;
@@ -916,7 +910,6 @@ bool run_fixed_no_alloc(const Problem &pb, cudaStream_t stream) {
   p.n_blocks = static_cast<int>((pb.N + BN - 1) / BN);
   p.num_tiles = m_blocks * p.n_blocks;
   p.num_kb = static_cast<int>((pb.K + BK - 1) / BK);
-  p.stages = Cfg::kStages;
   p.status = device_status_word_if_ready();
   HOM_DIAG(p.prof = nullptr; p.tl = nullptr;)
   p.split_k = 1;

@@ -418,5 +418,10 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
   return d;
 }
 
+// The descriptor of the operand `bytes` further on (a multiple of 16; same tile layout).
+__device__ __forceinline__ uint64_t smem_desc_advance(uint64_t desc, uint32_t bytes) {
+  return desc + (bytes >> 4);
+}
+
 }  // namespace ptx
 }  // namespace hom
