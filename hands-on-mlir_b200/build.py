@@ -38,6 +38,7 @@ RUNNER_SOURCES = [
     "context.cu",
     "gemm_sm100.cu",
     "gemm_pair_sm100.cu",
+    "gemm_cluster_sm100.cu",
     "attention_sm100.cu",
     "attention_pingpong_sm100.cu",
     "bandwidth_kernels.cu",

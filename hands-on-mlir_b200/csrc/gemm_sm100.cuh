@@ -74,6 +74,12 @@ bool layernorm_fusion_shape(int64_t n, int *cluster_n, int *bn);
 // The CTA-pair kernels (gemm_pair_sm100.cu); bn2 is 128 or 256.
 bool run_pair(const Problem &pb, int bn2, int split_k, cudaStream_t stream);
 
+// One cluster of `parts` CTAs per 128 x {64,128} tile, K split over the cluster
+// (gemm_cluster_sm100.cu); cluster_supported says whether `pb` can run on it.
+constexpr int kMaxClusterParts = 8;
+bool cluster_supported(const Problem &pb, int parts);
+bool run_cluster(const Problem &pb, int bn, int parts, cudaStream_t stream);
+
 // The 128 x 128 single-CTA kernel for `pb` (B as [K, N]) launched without any allocation (no
 // tensor-map cache insert, no status-word creation).
 bool run_fixed_no_alloc(const Problem &pb, cudaStream_t stream);

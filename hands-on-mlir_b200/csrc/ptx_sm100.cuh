@@ -306,6 +306,16 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
+// The two halves of the cluster barrier, for code that has work between them.  Each thread of
+// the cluster arrives and waits exactly once per phase.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // shared::cluster address of the same shared-memory offset in CTA `cta_rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta_rank) {
   uint32_t r;
