@@ -107,8 +107,8 @@ constexpr int kSplitSlotFloats = 32 * 64;
 // 64-column block per warp instead of two.  Each warp stages its [32 rows x 64 fp16 columns]
 // block in one 128-byte-swizzled tile that a TMA store then writes out.
 constexpr int kEpilogueWarps = 16;
-// Warp 0 is the TMA producer, warp 1 issues the MMAs, the epilogue warps follow.
-constexpr int kControlWarps = 2;
+// Warp 0 fetches A, warp 1 issues the MMAs, warp 2 fetches B, the epilogue warps follow.
+constexpr int kControlWarps = 3;
 constexpr uint32_t kEpilogueTileBytes = 32 * 128;
 constexpr uint32_t kEpilogueStageBytes = kEpilogueTileBytes;
 constexpr uint32_t kEpilogueStagingBytes = kEpilogueWarps * kEpilogueStageBytes;

@@ -7,9 +7,9 @@
 // shared memory for the same MMA time, which is what the TMA ring needs to keep the tensor
 // pipe fed; the freed shared memory holds five stages and the epilogue staging.
 //
-//   warp 0      TMA producer
+//   warps 0, 2  TMA producers of A and of B
 //   warp 1      tensor-memory allocation (both CTAs) and MMA issue (even CTA only)
-//   warps 2-17  epilogue: four warps per tensor-memory lane quarter, each draining one
+//   warps 3-18  epilogue: four warps per tensor-memory lane quarter, each draining one
 //               64-column group of the tile: tcgen05.ld, fp32 alpha/beta/bias/erf-GELU, fp16
 //               results staged in swizzled shared memory and written out by TMA stores
 //
@@ -64,6 +64,14 @@ struct PairParams {
   HOM_DIAG(long long *prof;)  // optional per-role cycle counters of CTA 0, else null
   HOM_DIAG(long long *tl;)    // optional launch-timeline slot, else null
 };
+
+// After an expired wait: gives copies already in flight time to land (about 2 ms) before the
+// CTA's shared memory is released.
+__device__ __forceinline__ void drain_copies() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 4000000LL) {
+  }
+}
 
 template <int BN2, bool B_NK, bool SPLIT = false, int FORMS = 0, int EPI = 0>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -133,11 +141,11 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   })
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    // One elected lane runs the whole loop (see gemm_sm100.cu).
+    // ------------------------------------------------------------ TMA producer, A
+    // One elected lane runs the whole loop; A and B come from two warps (see gemm_sm100.cu).
     if (elect_one()) {
-      // Copies of both CTAs complete on the even CTA's barriers, which the even CTA's producer
-      // arms for the bytes of both; `bar` is the stage's barrier in the even CTA (cluster address).
+      // Copies of both CTAs complete on the even CTA's barriers, which the even CTA's A producer
+      // arms for the bytes of all four (copies may land first: the phase needs the arrival).
       const uint32_t full_even = map_to_cta(full_bar(0), 0);
       uint32_t dst = smem_base, slot = 0, ph = 0;
       bool ok = true;
@@ -151,46 +159,22 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           ph ^= 1u;
         }
       };
-      const bool b_grouped = p.b_grouped != 0;
-      auto load_b = [&](uint32_t b_dst, uint32_t bar, int k, int nb0) {
-        if (B_NK) {
-          tma_load_2d_pair(b_dst, &tmB, bar, k, nb0);
-        } else if (b_grouped) {
-          tma_load_3d_pair(b_dst, &tmB, bar, 0, k, nb0 / 64);
-        } else {
-#pragma unroll
-          for (int g = 0; g < HALF / 64; ++g) tma_load_2d_pair(b_dst + g * (BK * 128), &tmB, bar, nb0 + g * 64, k);
-        }
-      };
-      // When B is a declared constant (weights, which no kernel of the stream writes) the
-      // first ring of B tiles is requested before waiting for the previous kernel; A, and a B
-      // of unknown origin, only after.
-      int pre = 0;
-      if (p.b_early && pair < p.num_units) {
-        const int tile0 = pair / p.split_k, part0 = pair % p.split_k;
-        const int nb0 = (tile0 % p.n_blocks) * BN2 + static_cast<int>(rank) * HALF;
-        const int kb0 = part0 * p.num_kb / p.split_k, kb1 = (part0 + 1) * p.num_kb / p.split_k;
-        pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
-        for (int i = 0; i < pre; ++i) {
-          if (rank == 0) mbar_arrive_expect_tx(full_bar(i), 2 * Cfg::kStageBytes);
-          load_b(smem_base + i * Cfg::kStageBytes + kABytes, full_even + 8u * i, (kb0 + i) * BK, nb0);
-        }
+      // The first ring is armed before the wait for the previous kernel (gemm_sm100.cu).
+      int ready = 0;
+      if (pair < p.num_units) {
+        const int part0 = pair % p.split_k;
+        ready = min(STAGES, (part0 + 1) * p.num_kb / p.split_k - part0 * p.num_kb / p.split_k);
+        if (rank == 0)
+          for (int i = 0; i < ready; ++i) mbar_arrive_expect_tx(full_bar(i), 2 * Cfg::kStageBytes);
       }
-      // longest entry -> first weight tiles requested (just before the dependency wait), ns
-      HOM_DIAG(if (p.tl) {
-        unsigned long long t;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        atomicMax(p.tl + 481, static_cast<long long>(t - g_entry));
-      })
       pdl_wait();
       HOM_DIAG(if (p.tl) timeline_stamp(p.tl, 2);)
       for (int unit = pair; unit < p.num_units && ok; unit += num_pairs) {
         const int tile = unit / p.split_k, part = unit % p.split_k;
         const int m0 = (tile / p.n_blocks) * 256 + static_cast<int>(rank) * 128;
-        const int nb0 = (tile % p.n_blocks) * BN2 + static_cast<int>(rank) * HALF;
-        int k = part * p.num_kb / p.split_k * BK;
         const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
-        for (; pre > 0; --pre, k += BK) {  // (first unit only: the B half is on its way)
+        int k = part * p.num_kb / p.split_k * BK;
+        for (; ready > 0; --ready, k += BK) {
           tma_load_2d_pair(dst, &tmA, full_even + slot, k, m0);
           advance();
         }
@@ -201,7 +185,6 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
           if (rank == 0) mbar_arrive_expect_tx(full_bar(0) + slot, 2 * Cfg::kStageBytes);
           tma_load_2d_pair(dst, &tmA, full_even + slot, k, m0);
-          load_b(dst + kABytes, full_even + slot, k, nb0);
           advance();
         }
       }
@@ -209,12 +192,44 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         p.prof[0 + 8 * blockIdx.x] = clock64() - t_begin;
         p.prof[1 + 8 * blockIdx.x] = t_wait;
       })
-      if (!ok) {
-        // Give copies already in flight time to land before shared memory is released.
-        const long long t0 = clock64();
-        while (clock64() - t0 < 4000000LL) {
+      if (!ok) drain_copies();
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ TMA producer, B
+    if (elect_one()) {
+      const uint32_t full_even = map_to_cta(full_bar(0), 0);
+      uint32_t dst = smem_base + kABytes, slot = 0, ph = 0;
+      bool ok = true;
+      const bool b_grouped = p.b_grouped != 0;
+      // A declared constant is requested without waiting for the previous kernel (gemm_sm100.cu).
+      if (!p.b_early) pdl_wait();
+      for (int unit = pair; unit < p.num_units && ok; unit += num_pairs) {
+        const int tile = unit / p.split_k, part = unit % p.split_k;
+        const int nb0 = (tile % p.n_blocks) * BN2 + static_cast<int>(rank) * HALF;
+        const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
+        for (int k = part * p.num_kb / p.split_k * BK; k < k_end; k += BK) {
+          ok = mbar_wait(empty_bar(0) + slot, ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutProducer);
+          if (!ok) break;
+          if (B_NK) {
+            tma_load_2d_pair(dst, &tmB, full_even + slot, k, nb0);
+          } else if (b_grouped) {
+            tma_load_3d_pair(dst, &tmB, full_even + slot, 0, k, nb0 / 64);
+          } else {
+#pragma unroll
+            for (int g = 0; g < HALF / 64; ++g)
+              tma_load_2d_pair(dst + g * (BK * 128), &tmB, full_even + slot, nb0 + g * 64, k);
+          }
+          dst += Cfg::kStageBytes;
+          slot += 8;
+          if (slot == 8 * STAGES) {
+            dst = smem_base + kABytes;
+            slot = 0;
+            ph ^= 1u;
+          }
         }
       }
+      if (!ok) drain_copies();
     }
     __syncwarp();
   } else if (warp == 1) {

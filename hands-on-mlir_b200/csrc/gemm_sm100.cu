@@ -2,12 +2,12 @@
 // tensor memory, Row,Row,Row operands (B as [K,N]) or the "transb" form (B as [N,K]).
 //
 // One persistent CTA per SM walks a static list of work units: a 128 x BN output tile, or one
-// of the `split_k` K ranges of a tile.  Inside a CTA (576 threads):
-//   warp 0      TMA producer: 128x64 A box + BN x 64 B boxes per K block into a ring of
+// of the `split_k` K ranges of a tile.  Inside a CTA (608 threads):
+//   warps 0, 2  TMA producers: 128x64 A box / BN x 64 B boxes per K block into a ring of
 //               128-byte-swizzled shared-memory stages (mbarrier full/empty hand-off);
 //   warp 1      issues tcgen05.mma (M=128, N=BN, K=16) into one of two TMEM accumulators and
 //               releases stages / publishes accumulators with tcgen05.commit;
-//   warps 2-17  epilogue (four warps per tensor-memory lane quarter, one 64-column group of
+//   warps 3-18  epilogue (four warps per tensor-memory lane quarter, one 64-column group of
 //               the tile each): tcgen05.ld the finished accumulator (one output row per
 //               thread, 32 columns at a time), fp32 alpha/beta/bias/erf-GELU, one fp16
 //               rounding, results staged in swizzled shared memory and written out by TMA
@@ -75,11 +75,11 @@ struct Params {
   int ln_cluster;
 };
 
-// Wait that ignores the CTA abort flag; used only to let in-flight TMA land before exit.
-__device__ __forceinline__ void mbar_wait_drain(uint32_t bar, uint32_t parity) {
+// After an expired wait: gives copies already in flight time to land (about 2 ms) before the
+// CTA's shared memory is released.
+__device__ __forceinline__ void drain_copies() {
   const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (clock64() - t0 > 200000000LL) break;
+  while (clock64() - t0 < 4000000LL) {
   }
 }
 
@@ -145,12 +145,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   HOM_DIAG(if (p.prof && blockIdx.x == 0 && threadIdx.x == 0) p.prof[10] = clock64() - t_entry;)
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    // One elected lane runs the whole loop (see the MMA issuer).
+    // ------------------------------------------------------------ TMA producer, A
+    // One elected lane runs the whole loop (see the MMA issuer).  A and B come from two warps: one
+    // thread that waits, arms and issues both copies needs about 280 clk per K block, more than
+    // the tensor pipe takes for a tile up to 128 columns wide.
     if (elect_one()) {
-      // The loop below is a chain of dependent instructions of one thread: addresses advance by
-      // additions, everything else is hoisted (40 clk a K block that the tensor pipe would wait).
-      uint32_t dst = smem_base, bar = full_bar(0), ph = 0, armed = 0;
+      // A chain of dependent instructions of one thread: addresses advance by additions.
+      uint32_t dst = smem_base, bar = full_bar(0), ph = 0;
       bool ok = true;
       HOM_DIAG(long long t_wait = 0; const long long t_begin = clock64();)
       auto advance = [&]() {
@@ -162,42 +163,23 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           ph ^= 1u;
         }
       };
-      const bool b_grouped = p.b_grouped != 0;
-      auto load_b = [&](uint32_t b_dst, uint32_t b_bar, int k, int n0) {
-        if (B_NK) {
-          tma_load_2d(b_dst, &tmB, b_bar, k, n0);
-        } else if (b_grouped) {
-          tma_load_3d(b_dst, &tmB, b_bar, 0, k, n0 / 64);
-        } else {
-#pragma unroll
-          for (int g = 0; g < BN / 64; ++g) tma_load_2d(b_dst + g * (BK * 128), &tmB, b_bar, n0 + g * 64, k);
-        }
-      };
-      // When B is a declared constant (weights, which no kernel of the stream writes) the
-      // first ring of B tiles is requested before waiting for the previous kernel; A, and a B
-      // of unknown origin, only after.
-      int pre = 0;
-      if (p.b_early && blockIdx.x < p.num_units) {
-        const int tile0 = blockIdx.x / p.split_k, part0 = blockIdx.x % p.split_k;
-        const int n0 = (tile0 % p.n_blocks) * BN;
-        const int kb0 = part0 * p.num_kb / p.split_k, kb1 = (part0 + 1) * p.num_kb / p.split_k;
-        pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
-        for (int i = 0; i < pre; ++i) {
-          mbar_arrive_expect_tx(full_bar(i), Cfg::kStageBytes);
-          load_b(smem_base + i * Cfg::kStageBytes + kABytes, full_bar(i), (kb0 + i) * BK, n0);
-        }
+      // The first ring is armed (for the bytes of both copies) before the wait for the previous
+      // kernel, so that only the copies themselves are left to do after it.
+      int ready = 0;
+      if (blockIdx.x < p.num_units) {
+        const int part0 = blockIdx.x % p.split_k;
+        ready = min(STAGES, (part0 + 1) * p.num_kb / p.split_k - part0 * p.num_kb / p.split_k);
+        for (int i = 0; i < ready; ++i) mbar_arrive_expect_tx(full_bar(i), Cfg::kStageBytes);
       }
       pdl_wait();
       HOM_DIAG(if (p.tl) timeline_stamp(p.tl, 2);)
       for (int unit = blockIdx.x; unit < p.num_units && ok; unit += gridDim.x) {
         const int tile = unit / p.split_k, part = unit % p.split_k;
         const int m0 = (tile / p.n_blocks) * BM;
-        const int n0 = (tile % p.n_blocks) * BN;
-        int k = part * p.num_kb / p.split_k * BK;
         const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
-        for (; pre > 0; --pre, k += BK) {  // (first unit only: the B half is on its way)
+        int k = part * p.num_kb / p.split_k * BK;
+        for (; ready > 0; --ready, k += BK) {
           tma_load_2d(dst, &tmA, bar, k, m0);
-          ++armed;
           advance();
         }
         for (; k < k_end; k += BK) {
@@ -207,8 +189,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           HOM_DIAG(if (p.prof) t_wait += clock64() - tw;)
           mbar_arrive_expect_tx(bar, Cfg::kStageBytes);
           tma_load_2d(dst, &tmA, bar, k, m0);
-          load_b(dst + kABytes, bar, k, n0);
-          ++armed;
           advance();
         }
       }
@@ -216,16 +196,49 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         p.prof[0] = clock64() - t_begin;
         p.prof[1] = t_wait;
       })
-      if (!ok) {
-        // Let every copy this warp started land before the CTA gives its shared memory back.
-        for (int st = 0; st < STAGES; ++st) {
-          const uint32_t n_st = armed / STAGES + (static_cast<uint32_t>(st) < armed % STAGES ? 1u : 0u);
-          if (n_st > 0) mbar_wait_drain(full_bar(st), (n_st - 1u) & 1u);
-        }
-      }
+      if (!ok) drain_copies();
     }
     __syncwarp();
     if constexpr (LN) cluster_sync_all();  // the epilogue's statistics exchange counts every thread
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ TMA producer, B
+    if (elect_one()) {
+      uint32_t dst = smem_base + kABytes, bar = full_bar(0), ph = 0;
+      bool ok = true;
+      const bool b_grouped = p.b_grouped != 0;
+      // A declared constant (weights, which no kernel of the stream writes) is requested without
+      // waiting for the previous kernel: the first ring of B tiles then arrives while that one
+      // finishes.  A B of unknown origin only after.  (Its bytes may land before the A warp has
+      // armed the barrier: the phase cannot complete without that arrival.)
+      if (!p.b_early) pdl_wait();
+      for (int unit = blockIdx.x; unit < p.num_units && ok; unit += gridDim.x) {
+        const int tile = unit / p.split_k, part = unit % p.split_k;
+        const int n0 = (tile % p.n_blocks) * BN;
+        const int k_end = (part + 1) * p.num_kb / p.split_k * BK;
+        for (int k = part * p.num_kb / p.split_k * BK; k < k_end; k += BK) {
+          ok = mbar_wait(bar + 8u * STAGES, ph ^ 1u, abort_flag, p.status, kDevWaitTimeoutProducer);
+          if (!ok) break;
+          if (B_NK) {
+            tma_load_2d(dst, &tmB, bar, k, n0);
+          } else if (b_grouped) {
+            tma_load_3d(dst, &tmB, bar, 0, k, n0 / 64);
+          } else {
+#pragma unroll
+            for (int g = 0; g < BN / 64; ++g) tma_load_2d(dst + g * (BK * 128), &tmB, bar, n0 + g * 64, k);
+          }
+          dst += Cfg::kStageBytes;
+          bar += 8;
+          if (bar == full_bar(STAGES)) {
+            dst = smem_base + kABytes;
+            bar = full_bar(0);
+            ph ^= 1u;
+          }
+        }
+      }
+      if (!ok) drain_copies();
+    }
+    __syncwarp();
+    if constexpr (LN) cluster_sync_all();
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
     // One lane, elected once by elect.sync around the whole loop: the compiler then knows that a
