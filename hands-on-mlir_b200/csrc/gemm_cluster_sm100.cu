@@ -14,6 +14,8 @@
 // rows.  Nothing goes through global scratch, and no CTA waits for another launch's counter.
 //
 // 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 accumulator exchange + epilogue.
+#include <atomic>
+
 #include <cuda_fp16.h>
 
 #include "gemm_epilogue.cuh"
@@ -370,6 +372,48 @@ bool launch_cluster(const Problem &pb, int parts, cudaStream_t stream) {
 bool cluster_supported(const Problem &pb, int parts) {
   return parts >= 2 && parts <= kMaxClusterParts && pb.N % 8 == 0 && parts <= (pb.K + BK - 1) / BK &&
          !has_layernorm_form(pb);
+}
+
+int cluster_capacity(int bn, int parts) {
+  // Clusters of more than two CTAs need SMs of one GPC; how many fit depends on which SMs of each
+  // GPC the device has.  Asked once per device; the fallback is a 148-SM part (and what a build
+  // machine without a GPU answers).
+  constexpr int kFallback[kMaxClusterParts + 1] = {0, 148, 74, 45, 33, 24, 18, 16, 14};
+  if (parts < 2 || parts > kMaxClusterParts) return 0;
+  static std::atomic<int> cache[64][2][kMaxClusterParts + 1] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    cudaGetLastError();
+    return kFallback[parts];
+  }
+  std::atomic<int> &slot = cache[dev][bn == 64 ? 0 : 1][parts];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  auto query = [&](auto kernel, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(parts);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(parts);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return count;
+  };
+  n = bn == 64 ? query(gemm_f16_cluster_kernel<64, false>, ClusterCfg<64>::kSmemBytes)
+               : query(gemm_f16_cluster_kernel<128, false>, ClusterCfg<128>::kSmemBytes);
+  if (n <= 0) n = kFallback[parts];
+  slot.store(n, std::memory_order_relaxed);
+  return n;
 }
 
 bool run_cluster(const Problem &pb, int bn, int parts, cudaStream_t stream) {

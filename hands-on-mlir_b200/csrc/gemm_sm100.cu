@@ -18,6 +18,7 @@
 // (include/NVGPUKernels/GemmRunner.h:119-310, lib/NVGPUKernels/GemmProfiler.cu:143-236) with a
 // small per-shape tile table.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstdio>
 #include <tuple>
@@ -794,13 +795,6 @@ bool launch_ln_variant(const Problem &pb, float eps, cudaStream_t stream) {
                     "gemm + layernorm kernel launch");
 }
 
-struct ShapeRow {
-  int64_t m, n, k;
-  int act;
-  int row;
-  int split;
-};
-
 // Tile-table rows: 1-4 = one CTA per 128 x {64,128,192,256} tile; 5, 6 = one CTA pair per
 // 256 x {128,256} tile.
 struct TileRow {
@@ -812,16 +806,6 @@ const TileRow kTileRows[7] = {
     {128, 256, 3, false},  {256, 128, 6, true},  {256, 256, 5, true},
 };
 constexpr int kNumTileRows = 6;
-
-// Per-shape choices for the BERT-base encoder GEMMs (M = batch*seq rows), replacing the
-// reference's autotune cache keyed on (M, N, K, activation).
-const ShapeRow kShapeTable[] = {
-    {4096, 2304, 768, 0, 6, 1},   // base QKV
-    {4096, 768, 768, 0, 3, 1},    // base attention output projection (+ residual)
-    {4096, 3072, 768, 1, 6, 1},   // base FFN1 + GELU
-    {4096, 768, 3072, 0, 3, 1},   // base FFN2 (+ residual)
-    {512, 3072, 768, 1, 2, 1},    // single fused GEMM + bias + GELU case
-};
 
 }  // namespace
 
@@ -1124,54 +1108,53 @@ bool tune(int64_t m, int64_t n, int64_t k, int act, float alpha, float beta, boo
 }
 
 namespace {
-// Estimated duration (clock cycles) of a launch with tile-table row `row` and K split `sp`.
-//   per K block: the slower of the MMA time (N / 2 clocks per 16-deep MMA on one SM) and the
-//   time to pull the block's operand bytes through the L2 -> SM path (~70 B/clk/SM);
-//   per unit: its K blocks plus whatever of the previous unit's epilogue they do not hide;
-//   per launch: the ramp (set-up, first loads) and the last unit's epilogue; a split adds the
-//   partial write / read round of the fix-up.
-double estimate_cycles(int row, int sp, int64_t m, int64_t n, int64_t k, int act) {
+// Estimated duration (microseconds, inside a chain of dependent launches) of a launch with
+// tile-table row `row` and K split `sp`.  The constants are a fit to 1,500 launches measured on
+// the GEMMs of both BERT sizes at M = 64 .. 16384 (rms 7-8 % per row; over those shapes the row
+// the estimate picks is on average 0.5 %, at worst 14 %, slower than the fastest one measured):
+//   whole-K tiles     fixed + rounds * K blocks * time per K block, which grows with the share of
+//                     the chip in use (the CTAs share the L2 -> SM path and the power budget),
+//                     plus what an epilogue outlasts the next tile's main loop by;
+//   clusters (rows 1 and 2 with a split of 2..8)   fixed + K blocks per CTA * time per block +
+//                     exchange, which grows with the parts and with the CTAs that exchange.
+struct RowCost {
+  double fixed, per_kb, epilogue, busy_kb, busy;
+};
+constexpr RowCost kRowCost[7] = {
+    {0, 0, 0, 0, 0},
+    {3.48, 0.181, 2.72, 0.135, 0.09},  // 128 x 64
+    {3.88, 0.202, 3.58, 0.303, 0.00},  // 128 x 128
+    {4.09, 0.273, 4.64, 0.267, 0.00},  // 128 x 192
+    {4.20, 0.394, 6.11, 0.210, 0.08},  // 128 x 256
+    {4.32, 0.193, 3.24, 0.280, 0.78},  // pair 256 x 128
+    {5.36, 0.283, 4.86, 0.320, 0.54},  // pair 256 x 256
+};
+
+double estimate_us(int row, int sp, int64_t m, int64_t n, int64_t k) {
   const TileRow &t = kTileRows[row];
-  const int sms = sm_count();
-  const int64_t tiles = ((m + t.tile_m - 1) / t.tile_m) * ((n + t.tile_n - 1) / t.tile_n);
-  const int64_t slots = t.pair ? sms / 2 : sms;
-  const int64_t num_kb = (k + BK - 1) / BK;
-  const int64_t units = tiles * sp;
-  const int64_t rounds = (units + slots - 1) / slots;
-  const double kb_unit = static_cast<double>((num_kb + sp - 1) / sp);
-  const double cols_per_sm = t.pair ? t.tile_n / 2.0 : t.tile_n;
-  const double bytes_kb = 128.0 * BK * 2 + cols_per_sm * BK * 2;
-  const double mma_kb = 4.0 * (t.tile_n < 128 ? 74.0 : t.tile_n / 2.0);
-  const double t_kb = std::max(mma_kb * 1.08, bytes_kb / 70.0);
-  const double t_epi = 1200.0 + (act ? 14.0 : 7.0) * t.tile_n;
-  const double t_unit = kb_unit * t_kb;
-  double cycles = 3000.0 + rounds * t_unit + (rounds - 1) * std::max(0.0, t_epi - t_unit) + t_epi;
-  // A split moves every unit's fp32 block through L2 once more per part (the same L2 -> SM
-  // path the operands use) and chains the parts' epilogues: measured 6-8 us per extra part at
-  // 256-wide tiles when the SMs are busy, so it only pays when most SMs would otherwise idle.
-  if (sp > 1) cycles += (sp - 1) * (3000.0 + 40.0 * cols_per_sm);
-  return cycles;
+  const double tiles = static_cast<double>(((m + t.tile_m - 1) / t.tile_m) * ((n + t.tile_n - 1) / t.tile_n));
+  const double num_kb = static_cast<double>((k + BK - 1) / BK);
+  if (sp > 1 && row <= 2 && sp <= kMaxClusterParts) {
+    const double kb = std::ceil(num_kb / sp);
+    return row == 1 ? 3.9 + 0.16 * kb + 0.13 * (sp - 2) + 0.006 * tiles * sp
+                    : 5.6 + 0.20 * kb + 0.10 * (sp - 2) + 0.005 * tiles * sp;
+  }
+  const RowCost &c = kRowCost[row];
+  const double slots = t.pair ? sm_count() / 2 : sm_count();
+  const double rounds = std::ceil(tiles * sp / slots);
+  const double share = std::min(tiles * sp, slots) / slots;
+  const double unit = std::ceil(num_kb / sp) * c.per_kb * (1.0 + c.busy_kb * share * share);
+  double us = c.fixed + rounds * unit + (rounds - 1) * std::max(0.0, c.epilogue - unit) + c.busy * share;
+  // The serial split (any other row or factor): every part moves its fp32 block through L2 once
+  // more and the parts' epilogues form a chain, 6-8 us per extra part at 256-wide tiles.
+  if (sp > 1) us += (sp - 1) * (1.6 + 0.02 * t.tile_n);
+  return us;
 }
 }  // namespace
 
-int select_split(int row, int64_t m, int64_t n, int64_t k, int act) {
-  if (row < 1 || row > kNumTileRows) return 1;
-  int splits[8];
-  const int n_splits = split_candidates(k, splits);
-  int best = 1;
-  double best_cost = 1e300;
-  for (int i = 0; i < n_splits; ++i) {
-    const double c = estimate_cycles(row, splits[i], m, n, k, act);
-    if (c < best_cost * 0.97) {  // a split has to pay for itself clearly
-      best_cost = c;
-      best = splits[i];
-    }
-  }
-  return best;
-}
-
-int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k) {
+int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k, bool may_split) {
   if (split_k) *split_k = 1;
+  const bool whole_n = may_split && n % 8 == 0;  // what the cluster form asks for
   HOM_DIAG(if (const char *env = std::getenv("HOM_GEMM_TILE")) {  // experiment knob
     const int v = std::atoi(env);
     if (v >= 1 && v <= kNumTileRows) {
@@ -1184,11 +1167,6 @@ int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k) {
     if (split_k) *split_k = sp;
     return row;
   }
-  for (const ShapeRow &r : kShapeTable)
-    if (r.m == m && r.n == n && r.k == k && r.act == act) {
-      if (split_k) *split_k = r.split;
-      return r.row;
-    }
   int best = 1, best_sp = 1;
   double best_cost = 1e300;
   int splits[8];
@@ -1196,15 +1174,18 @@ int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k) {
   for (int r = 1; r <= kNumTileRows; ++r) {
     const TileRow &t = kTileRows[r];
     const int64_t tiles = ((m + t.tile_m - 1) / t.tile_m) * ((n + t.tile_n - 1) / t.tile_n);
-    const int64_t slots = t.pair ? sm_count() / 2 : sm_count();
     for (int i = 0; i < n_splits; ++i) {
-      // split only a problem that leaves at least half of the SMs idle and has a long K
-      if (splits[i] > 1 && (2 * tiles > slots || k < 2048)) continue;
-      double c = estimate_cycles(r, splits[i], m, n, k, act);
+      const int parts = splits[i];
+      // Only the cluster form splits by itself, and only while all clusters run at once: a second
+      // wave of them costs 5 us, more than any split gains (36 clusters of 4, of which 33 fit:
+      // 8.3 us against 4.3 us for 36 clusters of 2).
+      if (parts > 1 && (!whole_n || r > 2 || parts > kMaxClusterParts || tiles > cluster_capacity(t.tile_n, parts)))
+        continue;
+      const double c = estimate_us(r, parts, m, n, k);
       if (c < best_cost - 1e-9) {
         best_cost = c;
         best = r;
-        best_sp = splits[i];
+        best_sp = parts;
       }
     }
   }
@@ -1263,7 +1244,7 @@ bool run(const Problem &pb, int tile_row, cudaStream_t stream) {
   if (pb.M == 0 || pb.N == 0) return true;
   int split = 1;
   if (tile_row < 1 || tile_row > kNumTileRows) {
-    tile_row = select_tile_row(pb.M, pb.N, pb.K, pb.act, &split);
+    tile_row = select_tile_row(pb.M, pb.N, pb.K, pb.act, &split, !has_layernorm_form(pb));
     if (pb.split_k >= 2) split = pb.split_k;
   } else {
     split = pb.split_k >= 2 ? pb.split_k : 1;

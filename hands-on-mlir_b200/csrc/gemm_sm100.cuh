@@ -79,15 +79,16 @@ bool run_pair(const Problem &pb, int bn2, int split_k, cudaStream_t stream);
 constexpr int kMaxClusterParts = 8;
 bool cluster_supported(const Problem &pb, int parts);
 bool run_cluster(const Problem &pb, int bn, int parts, cudaStream_t stream);
+// How many clusters of `parts` CTAs the device runs at once (128 x bn tiles).
+int cluster_capacity(int bn, int parts);
 
 // The 128 x 128 single-CTA kernel for `pb` (B as [K, N]) launched without any allocation (no
 // tensor-map cache insert, no status-word creation).
 bool run_fixed_no_alloc(const Problem &pb, cudaStream_t stream);
 
-// Tile-table row and K split for a shape (tuned entry, else table, else cost heuristic).
-int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k = nullptr);
-// Split the heuristic would use for a given row.
-int select_split(int row, int64_t m, int64_t n, int64_t k, int act);
+// Tile-table row and K split for a shape (tuned entry, else the cost estimate).  `may_split`
+// false: the problem only runs with whole-K tiles.
+int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k = nullptr, bool may_split = true);
 int query_tile(int64_t m, int64_t n, int64_t k, int act, int *bn, int *stages, int *split_k);
 
 // Run-time tuner (GemmProfiler's contract): times the tile-table rows for one shape, remembers
