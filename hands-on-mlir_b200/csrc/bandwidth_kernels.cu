@@ -246,7 +246,7 @@ row_stats_f16_kernel(const __half *x, __half *rstd_out, __half *shift_out, long 
 // (partials[g * rows + r] = {sum, sum of squares} of row r over columns [64 g, 64 g + 64)):
 // rstd = 1 / sqrt(E[x^2] - mean^2 + eps) and shift = -mean * rstd, stored as fp16 like the
 // reference's ApplyFinalReduction (include/NVGPUKernels/Layernorm.h:107-194).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(64)
 row_stats_finalize_kernel(const float2 *partials, int groups, long long rows, int n, float eps,
                           __half *rstd_out, __half *shift_out) {
   hom::ptx::pdl_launch_dependents();
@@ -254,6 +254,7 @@ row_stats_finalize_kernel(const float2 *partials, int groups, long long rows, in
   const long long r = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   float sum = 0.f, sq = 0.f;
+#pragma unroll 16
   for (int g = 0; g < groups; ++g) {
     const float2 v = partials[static_cast<long long>(g) * rows + r];
     sum += v.x;
@@ -282,24 +283,70 @@ repitch_rows_f16_kernel(const __half *src, __half *dst, long long rows, int cols
 }
 
 // out[n] = sum_k b[k, n] (b is [K, N]) or sum_k b[n, k] (b is [N, K]), fp32.
-__global__ void __launch_bounds__(256)
+// [K, N]: a block owns 64 columns, its 32 warps every 32nd row (two columns per lane, 128
+// contiguous bytes per warp and load, eight loads in flight), then the 32 partial sums of a column
+// are added in warp order.  Bound by latency: one thread per column walking all K rows took 46 us
+// at 768 x 3072, this form 3 us.
+// [N, K]: one warp per row of b, 16-byte loads where rows are aligned.
+constexpr int kColSumWarps = 32;
+
+__global__ void __launch_bounds__(32 * kColSumWarps)
 col_sum_f16_kernel(const __half *b, float *out, int k_dim, int n_dim, int b_is_nk) {
   hom::ptx::pdl_launch_dependents();
   hom::ptx::pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (b_is_nk) {
-    const int lane = threadIdx.x & 31;
-    const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int n = blockIdx.x * kColSumWarps + warp;
     if (n >= n_dim) return;
+    const __half *row = b + static_cast<long long>(n) * k_dim;
     float s = 0.f;
-    for (int k = lane; k < k_dim; k += 32) s += __half2float(b[static_cast<long long>(n) * k_dim + k]);
+    if ((k_dim & 7) == 0 && (reinterpret_cast<uintptr_t>(b) & 15u) == 0) {
+      const uint4 *v = reinterpret_cast<const uint4 *>(row);
+#pragma unroll 4
+      for (int i = lane; i < (k_dim >> 3); i += 32) {
+        const uint4 raw = v[i];
+        const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __half22float2(h2[j]);
+          s += f.x + f.y;
+        }
+      }
+    } else {
+      for (int k = lane; k < k_dim; k += 32) s += __half2float(row[k]);
+    }
     s = warp_sum(s);
     if (lane == 0) out[n] = s;
+    return;
+  }
+  __shared__ float2 part[kColSumWarps][32];
+  const int n = blockIdx.x * 64 + 2 * lane;
+  float2 s = make_float2(0.f, 0.f);
+  if ((n_dim & 1) == 0 && (reinterpret_cast<uintptr_t>(b) & 3u) == 0) {  // pairs are 4-byte aligned
+    if (n < n_dim) {
+#pragma unroll 8
+      for (int k = warp; k < k_dim; k += kColSumWarps) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(b + static_cast<long long>(k) * n_dim + n));
+        s.x += f.x;
+        s.y += f.y;
+      }
+    }
   } else {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= n_dim) return;
-    float s = 0.f;
-    for (int k = 0; k < k_dim; ++k) s += __half2float(b[static_cast<long long>(k) * n_dim + n]);
-    out[n] = s;
+    for (int k = warp; k < k_dim; k += kColSumWarps) {
+      const __half *p = b + static_cast<long long>(k) * n_dim + n;
+      if (n < n_dim) s.x += __half2float(p[0]);
+      if (n + 1 < n_dim) s.y += __half2float(p[1]);
+    }
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  // thread t < 64 adds up column t: part[w] seen as 64 consecutive floats
+  const int col = threadIdx.x;
+  if (col < 64 && blockIdx.x * 64 + col < n_dim) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kColSumWarps; ++w) t += reinterpret_cast<const float *>(part[w])[col];
+    out[blockIdx.x * 64 + col] = t;
   }
 }
 
@@ -646,8 +693,8 @@ bool row_stats_finalize(const float2 *partials, int groups, int64_t rows, int64_
                         __half *shift_out, cudaStream_t stream) {
   if (rows == 0) return true;
   LaunchScope scope(kOpLayernorm, 0.0, 8.0 * groups * rows + 4.0 * rows);
-  const unsigned blocks = static_cast<unsigned>((rows + 255) / 256);
-  return check_cuda(launch_pdl(row_stats_finalize_kernel, dim3(blocks), dim3(256), 0, stream, 1, partials, groups,
+  const unsigned blocks = static_cast<unsigned>((rows + 63) / 64);
+  return check_cuda(launch_pdl(row_stats_finalize_kernel, dim3(blocks), dim3(64), 0, stream, 1, partials, groups,
                                static_cast<long long>(rows), static_cast<int>(n), eps, rstd_out, shift_out),
                     "row statistics finaliser launch");
 }
@@ -666,9 +713,8 @@ bool col_sum_f16(const __half *b, float *out, int64_t k_dim, int64_t n_dim, bool
                  cudaStream_t stream) {
   if (n_dim == 0) return true;
   LaunchScope scope(kOpElementwise, 0.0, 2.0 * k_dim * n_dim + 4.0 * n_dim);
-  const unsigned blocks = b_is_nk ? static_cast<unsigned>((n_dim + 7) / 8)
-                                  : static_cast<unsigned>((n_dim + 255) / 256);
-  return check_cuda(launch_pdl(col_sum_f16_kernel, dim3(blocks), dim3(256), 0, stream, 1, b, out,
+  const unsigned blocks = static_cast<unsigned>(b_is_nk ? (n_dim + kColSumWarps - 1) / kColSumWarps : (n_dim + 63) / 64);
+  return check_cuda(launch_pdl(col_sum_f16_kernel, dim3(blocks), dim3(32 * kColSumWarps), 0, stream, 1, b, out,
                                static_cast<int>(k_dim), static_cast<int>(n_dim), b_is_nk ? 1 : 0),
                     "column sum kernel launch");
 }

@@ -166,22 +166,29 @@ void *derived_lookup(const void *ptr, int64_t k, int64_t n) {
   auto it = g_padded_weights.find(PaddedKey{reinterpret_cast<uintptr_t>(ptr), k, n});
   return it == g_padded_weights.end() ? nullptr : it->second;
 }
-void derived_insert(const void *ptr, int64_t k, int64_t n, void *data) {
+// Two threads may have derived the same thing at once: the first one's stays (the other thread may
+// already be launching with it), the later one is given back.  Returns what the store holds.
+void *derived_insert(const void *ptr, int64_t k, int64_t n, void *data) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
   void *&slot = g_padded_weights[PaddedKey{reinterpret_cast<uintptr_t>(ptr), k, n}];
-  if (slot) cudaFree(slot);
-  slot = data;
+  if (slot) cudaFree(data);
+  else slot = data;
+  return slot;
 }
 }  // namespace
 
 const __half *padded_weight_lookup(const void *ptr, int64_t k, int64_t n) {
   return static_cast<const __half *>(derived_lookup(ptr, k, n));
 }
-void padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy) { derived_insert(ptr, k, n, copy); }
+const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy) {
+  return static_cast<const __half *>(derived_insert(ptr, k, n, copy));
+}
 const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n) {
   return static_cast<const float *>(derived_lookup(ptr, k, -n));
 }
-void weight_colsum_insert(const void *ptr, int64_t k, int64_t n, float *sums) { derived_insert(ptr, k, -n, sums); }
+const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, float *sums) {
+  return static_cast<const float *>(derived_insert(ptr, k, -n, sums));
+}
 
 void declare_constant_range(const void *ptr, size_t bytes) {
   if (!ptr || bytes == 0) return;

@@ -390,9 +390,10 @@ bool repitch_unaligned_b(const char *name, hom::gemm::Problem *pb) {
         cudaFree(fresh);
         return false;
       }
-      hom::padded_weight_insert(pb->B, pb->K, pb->N, fresh);
+      copy = hom::padded_weight_insert(pb->B, pb->K, pb->N, fresh);
+    } else {
+      copy = fresh;
     }
-    copy = fresh;
   }
   (void)name;
   pb->B = copy;
@@ -430,6 +431,50 @@ float *col_sum_scratch() {
     bufs[dev] = static_cast<float *>(ptr);
   }
   return bufs[dev];
+}
+
+// The column sums of pb.B (fp32).  Those of a declared weight are computed once and kept until the
+// declaration is withdrawn or renewed, those of any other B on every call.  While the stream is
+// being captured nothing can be allocated or waited for, so sums that are not there yet are
+// computed into the scratch as part of the graph.  Null (error recorded) on failure.
+const float *column_sums(const char *name, const hom::gemm::Problem &pb, cudaStream_t stream) {
+  bool keep = pb.b_const;
+  if (keep) {
+    if (const float *sums = hom::weight_colsum_lookup(pb.B, pb.K, pb.N)) return sums;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      keep = false;
+    }
+  }
+  float *fresh = nullptr;
+  if (keep) {
+    void *ptr = nullptr;
+    if (!hom::check_cuda(cudaMalloc(&ptr, static_cast<size_t>(pb.N) * sizeof(float)), "cudaMalloc(column sums)"))
+      return nullptr;
+    fresh = static_cast<float *>(ptr);
+  } else {
+    if (pb.N > kColSumCapacity) {
+      set_error(HOM_ERR_UNSUPPORTED, "%s: N = %lld exceeds the %lld-column scratch", name,
+                static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
+      return nullptr;
+    }
+    fresh = col_sum_scratch();
+    if (!fresh) return nullptr;
+  }
+  if (!hom::bw::col_sum_f16(pb.B, fresh, pb.K, pb.N, pb.b_is_nk, stream)) {
+    if (keep) cudaFree(fresh);
+    return nullptr;
+  }
+  if (keep) {
+    // other streams may use the kept sums next: make them complete before they become visible
+    if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(column sums)")) {
+      cudaFree(fresh);
+      return nullptr;
+    }
+    return hom::weight_colsum_insert(pb.B, pb.K, pb.N, fresh);
+  }
+  return fresh;
 }
 
 // Var / Mean operands of the fused forms: rank-1 fp16 with at least `rows` entries.
@@ -648,12 +693,10 @@ void cutlassLayernormGemmF16(int64_t rankA, void *dstA, int64_t rankB, void *dst
               static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
     return;
   }
-  float *col_sum = col_sum_scratch();
-  if (!col_sum) return;
-  if (!hom::bw::col_sum_f16(pb.B, col_sum, pb.K, pb.N, false, hom::current_stream())) return;
   pb.row_scale = var;
   pb.row_shift = mean;
-  pb.col_sum = col_sum;
+  pb.col_sum = column_sums("cutlassLayernormGemmF16", pb, hom::current_stream());
+  if (!pb.col_sum) return;
   hom::gemm::run(pb, 0, hom::current_stream());
 }
 
@@ -802,38 +845,9 @@ void homGemmDeferredLayernormF16(int64_t rankA, void *dstA, int64_t rankStatsA, 
   }
   cudaStream_t stream = hom::current_stream();
   if (stats_a) {
-    // LayerNorm(A).B = rstd * (A.B) - mean * rstd * colsum(B): the column sums of a declared
-    // weight are computed once and kept, those of any other B on every call.
-    const float *sums = pb.b_const ? hom::weight_colsum_lookup(pb.B, pb.K, pb.N) : nullptr;
-    if (!sums) {
-      float *fresh = nullptr;
-      if (pb.b_const) {
-        void *ptr = nullptr;
-        if (!hom::check_cuda(cudaMalloc(&ptr, static_cast<size_t>(pb.N) * sizeof(float)), "cudaMalloc(column sums)"))
-          return;
-        fresh = static_cast<float *>(ptr);
-      } else {
-        if (pb.N > kColSumCapacity) {
-          set_error(HOM_ERR_UNSUPPORTED, "%s: N = %lld exceeds the %lld-column scratch", name,
-                    static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
-          return;
-        }
-        fresh = col_sum_scratch();
-        if (!fresh) return;
-      }
-      if (!hom::bw::col_sum_f16(pb.B, fresh, pb.K, pb.N, weightsNK, stream)) {
-        if (pb.b_const) cudaFree(fresh);
-        return;
-      }
-      if (pb.b_const) {
-        if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(column sums)")) {
-          cudaFree(fresh);
-          return;
-        }
-        hom::weight_colsum_insert(pb.B, pb.K, pb.N, fresh);
-      }
-      sums = fresh;
-    }
+    // LayerNorm(A).B = rstd * (A.B) - mean * rstd * colsum(B)
+    const float *sums = column_sums(name, pb, stream);
+    if (!sums) return;
     pb.col_sum = sums;
     pb.a_partials = stats_a;
     pb.a_groups = static_cast<int>(ga);
