@@ -201,6 +201,11 @@ __device__ __forceinline__ void epilogue_load_c(const EpilogueParams &ep, int ro
     const unsigned short *cu = reinterpret_cast<const unsigned short *>(cp);
 #pragma unroll
     for (int g = G0; g < G1; ++g) {
+      // A bias row starts 16-byte aligned whatever N is: only its last, ragged group is special.
+      if (ep.c_mode == 2 && (reinterpret_cast<uintptr_t>(cp) & 15u) == 0 && c0 + g * 8 + 8 <= ep.N) {
+        cval[g] = *reinterpret_cast<const uint4 *>(cp + g * 8);
+        continue;
+      }
       uint32_t w[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -457,7 +462,30 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
     __syncwarp();
     const int col = c0 + 2 * lane;
     const uint32_t chunk = static_cast<uint32_t>(lane) >> 2, within = (static_cast<uint32_t>(lane) & 3u) << 2;
-    for (int r = 0; r < 32; ++r) {
+    // Whole blocks with 4-byte aligned pairs (N even): eight rows in flight.  One row at a time -
+    // a shared-memory load, an alignment test and a store that wait for one another - made the
+    // drain of a 256-column tile twice as long as its main loop at K = 768.
+    const bool pairs = (ep.N & 1) == 0 && (reinterpret_cast<uintptr_t>(ep.D) & 3u) == 0;
+    const bool whole = pairs && c0 + 64 <= ep.N && row0 + 32 <= ep.M;
+    if (whole) {
+      __half *dp = ep.D + static_cast<long long>(row0) * ep.ldd + col;
+#pragma unroll
+      for (int r0 = 0; r0 < 32; r0 += 8) {
+        uint32_t word[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          asm volatile("ld.shared.b32 %0, [%1];"
+                       : "=r"(word[r])
+                       : "r"(stage_smem + (r0 + r) * 128 + ((chunk ^ static_cast<uint32_t>(r)) << 4) + within)
+                       : "memory");
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          *reinterpret_cast<uint32_t *>(dp) = word[r];
+          dp += ep.ldd;
+        }
+      }
+    }
+    for (int r = 0; r < 32 && !whole; ++r) {
       const int grow = row0 + r;
       if (grow >= ep.M) break;
       uint32_t word;
