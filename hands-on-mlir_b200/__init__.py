@@ -67,6 +67,9 @@ class MemRef:
             self._words[3 + i] = shape[i]
             self._words[3 + rank + i] = self.strides[i]
         self._keepalive = keepalive
+        # built once: the cast costs more than the rest of a call's argument conversion (it also
+        # keeps the words alive for a caller that only holds `args`)
+        self.args = c_int64(rank), ctypes.cast(self._words, c_void_p)
 
     @classmethod
     def of(cls, tensor) -> "MemRef":
@@ -83,10 +86,6 @@ class MemRef:
     @property
     def data_ptr(self) -> int:
         return int(self._words[1])
-
-    @property
-    def args(self):
-        return c_int64(self.rank), ctypes.cast(self._words, c_void_p)
 
 
 NULL_MEMREF = (c_int64(0), c_void_p(None))
@@ -218,20 +217,17 @@ class RunnerUtils:
         self.lib.homForgetWeights(c_void_p(tensor.data_ptr()))
 
     # ------------------------------------------------------------------ compute
-    def _gemm(self, fn, A, B, C, D, transa, transb, act, alpha, beta, gemm_num, split_k):
-        fn(*_as_args(A), transa, *_as_args(B), transb, *_as_args(C), *_as_args(D), act, alpha,
-           beta, gemm_num, split_k)
-        self.check()
-
     def cutlassGemmF16(self, A, B, C, D, activation=0, alpha=1.0, beta=0.0, gemmNum=0,
                        splitKFactor=1, transa=False, transb=False):
-        self._gemm(self.lib.cutlassGemmF16, A, B, C, D, transa, transb, activation, alpha, beta,
-                   gemmNum, splitKFactor)
+        self.lib.cutlassGemmF16(*_as_args(A), transa, *_as_args(B), transb, *_as_args(C), *_as_args(D),
+                                activation, alpha, beta, gemmNum, splitKFactor)
+        self.check()
 
     def nvteGemmF16(self, A, B, C, D, activation=0, alpha=1.0, beta=0.0, transa=False,
                     transb=True, gemmNum=0):
-        self._gemm(self.lib.nvteGemmF16, A, B, C, D, transa, transb, activation, alpha, beta,
-                   gemmNum, 0)
+        self.lib.nvteGemmF16(*_as_args(A), transa, *_as_args(B), transb, *_as_args(C), *_as_args(D),
+                             activation, alpha, beta, gemmNum, 0)
+        self.check()
 
     def cutlassGemmWithVarMeanF16(self, A, B, C, D, Var, Mean, alpha=1.0, beta=0.0, activation=0,
                                   eps=1e-5):

@@ -18,6 +18,7 @@
 // (include/NVGPUKernels/GemmRunner.h:119-310, lib/NVGPUKernels/GemmProfiler.cu:143-236) with a
 // small per-shape tile table.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -933,6 +934,7 @@ struct TuneChoice {
 };
 std::map<TuneKey, TuneChoice> g_tuned;
 std::mutex g_tuned_mutex;
+std::atomic<uint32_t> g_tuned_epoch{1};  // bumped after every change of g_tuned
 
 void load_env_cache_once() {
   static std::once_flag once;
@@ -997,6 +999,7 @@ int tune_cache_load(const char *path) {
     }
   }
   std::fclose(f);
+  g_tuned_epoch.fetch_add(1);
   return count;
 }
 
@@ -1100,6 +1103,7 @@ bool tune(int64_t m, int64_t n, int64_t k, int act, float alpha, float beta, boo
   {
     std::lock_guard<std::mutex> lock(g_tuned_mutex);
     g_tuned[TuneKey{m, n, k, act}] = TuneChoice{best, best_sp};
+    g_tuned_epoch.fetch_add(1);
   }
   if (best_row) *best_row = best;
   if (best_split) *best_split = best_sp;
@@ -1152,7 +1156,8 @@ double estimate_us(int row, int sp, int64_t m, int64_t n, int64_t k) {
 }
 }  // namespace
 
-int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k, bool may_split) {
+namespace {
+int choose_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k, bool may_split) {
   if (split_k) *split_k = 1;
   const bool whole_n = may_split && n % 8 == 0;  // what the cluster form asks for
   HOM_DIAG(if (const char *env = std::getenv("HOM_GEMM_TILE")) {  // experiment knob
@@ -1191,6 +1196,46 @@ int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k, bool
   }
   if (split_k) *split_k = best_sp;
   return best;
+}
+
+}  // namespace
+
+// A program calls with a handful of shapes over and over, and weighing 20 candidates takes longer
+// than the rest of a call: each thread keeps its latest choices, one per hash slot, valid for one
+// device until the table of tuned shapes changes.
+int select_tile_row(int64_t m, int64_t n, int64_t k, int act, int *split_k, bool may_split) {
+#if HOM_DIAG_ENABLED
+  return choose_tile_row(m, n, k, act, split_k, may_split);  // the experiment knobs may change between calls
+#else
+  struct Choice {
+    int64_t m = -1, n = 0, k = 0;
+    int act = 0, device = -1;
+    bool may_split = false;
+    uint32_t epoch = 0;
+    int row = 0, split = 1;
+  };
+  thread_local Choice recent[64];
+  load_env_cache_once();
+  const uint32_t epoch = g_tuned_epoch.load();
+  int device = 0;
+  cudaGetDevice(&device);
+  const uint64_t h = (static_cast<uint64_t>(m) * 0x9E3779B97F4A7C15ull) ^ (static_cast<uint64_t>(n) * 0xC2B2AE3D27D4EB4Full) ^
+                     (static_cast<uint64_t>(k) * 0x165667B19E3779F9ull) ^ static_cast<uint64_t>(2 * act + may_split);
+  Choice &c = recent[(h ^ (h >> 32)) >> 7 & 63];
+  if (c.m != m || c.n != n || c.k != k || c.act != act || c.may_split != may_split || c.device != device ||
+      c.epoch != epoch) {
+    c.row = choose_tile_row(m, n, k, act, &c.split, may_split);
+    c.m = m;
+    c.n = n;
+    c.k = k;
+    c.act = act;
+    c.may_split = may_split;
+    c.device = device;
+    c.epoch = epoch;
+  }
+  if (split_k) *split_k = c.split;
+  return c.row;
+#endif
 }
 
 int query_tile(int64_t m, int64_t n, int64_t k, int act, int *bn, int *stages, int *split_k) {
