@@ -646,8 +646,9 @@ namespace {
 struct OutMapKey {
   const void *ptr;
   uint64_t hidden, seq, bs;
+  uint32_t box_rows;
   bool operator==(const OutMapKey &o) const {
-    return ptr == o.ptr && hidden == o.hidden && seq == o.seq && bs == o.bs;
+    return ptr == o.ptr && hidden == o.hidden && seq == o.seq && bs == o.bs && box_rows == o.box_rows;
   }
 };
 struct OutMapKeyHash {
@@ -656,15 +657,17 @@ struct OutMapKeyHash {
     h = h * 1000003u ^ k.hidden;
     h = h * 1000003u ^ k.seq;
     h = h * 1000003u ^ k.bs;
+    h = h * 1000003u ^ k.box_rows;
     return h;
   }
 };
 
-// Output [bs, seq, hidden] fp16 as a 3-D tensor (hidden, seq, bs) with 64 x 128 x 1 boxes.
-bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, CUtensorMap *out) {
+}  // namespace
+
+bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, uint32_t box_rows, CUtensorMap *out) {
   static std::mutex mu;
   static std::unordered_map<OutMapKey, CUtensorMap, OutMapKeyHash> cache;
-  const OutMapKey key{ptr, hidden, seq, bs};
+  const OutMapKey key{ptr, hidden, seq, bs, box_rows};
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
@@ -687,7 +690,7 @@ bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, C
   }
   cuuint64_t dims[3] = {hidden, seq, bs};
   cuuint64_t strides[2] = {hidden * 2, hidden * seq * 2};
-  cuuint32_t box[3] = {kHeadDim, kTile, 1};
+  cuuint32_t box[3] = {kHeadDim, box_rows, 1};
   cuuint32_t elem[3] = {1, 1, 1};
   const CUresult r = reinterpret_cast<EncodeFn>(sym)(
       out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, elem,
@@ -703,7 +706,6 @@ bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, C
   return true;
 }
 
-}  // namespace
 
 bool run(const Problem &pb, cudaStream_t stream) {
   if (pb.bs == 0 || pb.seq == 0 || pb.heads == 0) return true;
@@ -762,7 +764,7 @@ bool run(const Problem &pb, cudaStream_t stream) {
       attr1_set[dev] = true;
     }
     CUtensorMap tm_out;
-    if (!make_out_map(pb.out, pb.heads * kHeadDim, pb.seq, pb.bs, &tm_out)) return false;
+    if (!make_out_map(pb.out, pb.heads * kHeadDim, pb.seq, pb.bs, kTile, &tm_out)) return false;
     const bool launched = check_cuda(launch_pdl(attention_f16_single_tile_kernel, grid, dim3(kThreads1),
                                                 kSmemBytes1, stream, 1, tm, tm_out, p),
                                      "attention kernel launch");

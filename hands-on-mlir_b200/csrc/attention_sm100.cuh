@@ -1,6 +1,8 @@
 // Host interface of the sm_100a packed-QKV attention kernel (attention_sm100.cu).
 #pragma once
 
+#include <cuda.h>
+
 #include "hom_common.cuh"
 
 namespace hom {
@@ -15,6 +17,8 @@ struct Problem {
 };
 
 bool run(const Problem &pb, cudaStream_t stream);
+// Output [bs, seq, hidden] fp16 as a cached 3-D tensor map (hidden, seq, bs) with 64 x box_rows x 1 boxes.
+bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, uint32_t box_rows, CUtensorMap *out);
 // seq > 128: the persistent kernel that owns two query tiles per CTA (attention_pingpong_sm100.cu).
 bool run_pingpong(const Problem &pb, cudaStream_t stream);
 
