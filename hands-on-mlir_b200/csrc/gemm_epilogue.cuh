@@ -111,7 +111,6 @@ constexpr int kEpilogueWarps = 16;
 constexpr int kControlWarps = 3;
 constexpr uint32_t kEpilogueTileBytes = 32 * 128;
 constexpr uint32_t kEpilogueStageBytes = kEpilogueTileBytes;
-constexpr uint32_t kEpilogueStagingBytes = kEpilogueWarps * kEpilogueStageBytes;
 
 // Bits of the FORMS mask of the GEMM kernels and of epilogue_warp_block.
 constexpr int kFormLnA = 1, kFormLnR = 2, kFormStats = 4;

@@ -41,9 +41,9 @@ struct PairCfg {
   static constexpr int kHalfN = BN2 / 2;
   static constexpr uint32_t kBBytes = kHalfN * BK * 2;
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = BN2 == 256 ? 5 : 6;
+  static constexpr int kStages = BN2 == 256 ? 5 : 8;
   static constexpr uint32_t kTmemCols = 2 * BN2;  // two accumulators; 512 or 256
-  static constexpr uint32_t kStagingBytes = kEpilogueStagingBytes;
+  static constexpr uint32_t kStagingBytes = BN2 / 64 * 4 * kEpilogueStageBytes;
   static constexpr uint32_t kBarrierBytes = 8 * (2 * kStages + 4) + 16;
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
 };

@@ -49,10 +49,10 @@ template <int BN>
 struct TileCfg {
   static constexpr uint32_t kBBytes = BN * BK * 2;
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  // As many stages as fit beside the 64 KB of epilogue staging.
-  static constexpr int kStages = BN == 256 ? 3 : BN == 192 ? 4 : BN == 128 ? 5 : 6;
+  // As many stages as fit beside the epilogue staging of the tile's BN / 64 column groups.
+  static constexpr int kStages = BN == 256 ? 3 : BN == 192 ? 4 : BN == 128 ? 6 : 8;
   static constexpr uint32_t kTmemCols = BN == 64 ? 128 : BN == 128 ? 256 : 512;
-  static constexpr uint32_t kStagingBytes = kEpilogueStagingBytes;
+  static constexpr uint32_t kStagingBytes = BN / 64 * 4 * kEpilogueStageBytes;
   static constexpr uint32_t kBarrierBytes = 8 * (2 * kStages + 4) + 16;
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
 };
@@ -803,8 +803,8 @@ struct TileRow {
   bool pair;
 };
 const TileRow kTileRows[7] = {
-    {0, 0, 0, false},      {128, 64, 6, false},  {128, 128, 5, false}, {128, 192, 4, false},
-    {128, 256, 3, false},  {256, 128, 6, true},  {256, 256, 5, true},
+    {0, 0, 0, false},      {128, 64, 8, false},  {128, 128, 6, false}, {128, 192, 4, false},
+    {128, 256, 3, false},  {256, 128, 8, true},  {256, 256, 5, true},
 };
 constexpr int kNumTileRows = 6;
 
@@ -1114,8 +1114,8 @@ bool tune(int64_t m, int64_t n, int64_t k, int act, float alpha, float beta, boo
 namespace {
 // Estimated duration (microseconds, inside a chain of dependent launches) of a launch with
 // tile-table row `row` and K split `sp`.  The constants are a fit to 1,500 launches measured on
-// the GEMMs of both BERT sizes at M = 64 .. 16384 (rms 7-8 % per row; over those shapes the row
-// the estimate picks is on average 0.5 %, at worst 14 %, slower than the fastest one measured):
+// the GEMMs of both BERT sizes at M = 64 .. 16384 (rms 6-8 % per row; over those shapes the row
+// the estimate picks is on average 0.4 %, at worst 8 %, slower than the fastest one measured):
 //   whole-K tiles     fixed + rounds * K blocks * time per K block, which grows with the share of
 //                     the chip in use (the CTAs share the L2 -> SM path and the power budget),
 //                     plus what an epilogue outlasts the next tile's main loop by;
@@ -1126,12 +1126,12 @@ struct RowCost {
 };
 constexpr RowCost kRowCost[7] = {
     {0, 0, 0, 0, 0},
-    {3.48, 0.181, 2.72, 0.135, 0.09},  // 128 x 64
-    {3.88, 0.202, 3.58, 0.303, 0.00},  // 128 x 128
-    {4.09, 0.273, 4.64, 0.267, 0.00},  // 128 x 192
-    {4.20, 0.394, 6.11, 0.210, 0.08},  // 128 x 256
-    {4.32, 0.193, 3.24, 0.280, 0.78},  // pair 256 x 128
-    {5.36, 0.283, 4.86, 0.320, 0.54},  // pair 256 x 256
+    {3.16, 0.181, 2.65, 0.087, 0.77},  // 128 x 64
+    {3.98, 0.182, 3.42, 0.383, 0.08},  // 128 x 128
+    {3.97, 0.273, 4.56, 0.249, 0.27},  // 128 x 192
+    {4.02, 0.396, 5.86, 0.168, 0.55},  // 128 x 256
+    {4.15, 0.193, 3.13, 0.217, 1.32},  // pair 256 x 128
+    {5.21, 0.286, 4.73, 0.268, 0.90},  // pair 256 x 256
 };
 
 double estimate_us(int row, int sp, int64_t m, int64_t n, int64_t k) {
@@ -1141,7 +1141,7 @@ double estimate_us(int row, int sp, int64_t m, int64_t n, int64_t k) {
   if (sp > 1 && row <= 2 && sp <= kMaxClusterParts) {
     const double kb = std::ceil(num_kb / sp);
     return row == 1 ? 3.9 + 0.16 * kb + 0.13 * (sp - 2) + 0.006 * tiles * sp
-                    : 5.6 + 0.20 * kb + 0.10 * (sp - 2) + 0.005 * tiles * sp;
+                    : 5.9 + 0.22 * kb + 0.10 * (sp - 2) + 0.005 * tiles * sp;
   }
   const RowCost &c = kRowCost[row];
   const double slots = t.pair ? sm_count() / 2 : sm_count();
