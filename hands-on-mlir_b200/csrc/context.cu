@@ -6,6 +6,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -150,44 +151,59 @@ bool split_workspace(size_t slot_floats, size_t blocks, cudaStream_t stream, Spl
 }
 
 namespace {
-struct PaddedKey {
+enum class Derived : int { kRepitched, kColumnSumsKN, kColumnSumsNK };
+struct DerivedKey {
   uintptr_t ptr;
-  int64_t k, n;  // n < 0: the entry holds the column sums of the [k, -n] weight
-  bool operator<(const PaddedKey &o) const {
-    return ptr != o.ptr ? ptr < o.ptr : k != o.k ? k < o.k : n < o.n;
+  int64_t k, n;
+  // What was derived.  A buffer can be read as [k, n] by one call and as [n, k] by another (a
+  // square weight), and its sums over k differ.
+  Derived kind;
+  bool operator<(const DerivedKey &o) const {
+    return std::tie(ptr, k, n, kind) < std::tie(o.ptr, o.k, o.n, o.kind);
   }
 };
-std::map<PaddedKey, void *> g_padded_weights;  // guarded by g_const_mutex
-}  // namespace
+std::map<DerivedKey, void *> g_derived;  // guarded by g_const_mutex
 
-namespace {
-void *derived_lookup(const void *ptr, int64_t k, int64_t n) {
+DerivedKey derived_key(const void *ptr, int64_t k, int64_t n, Derived kind) {
+  return DerivedKey{reinterpret_cast<uintptr_t>(ptr), k, n, kind};
+}
+Derived column_sums_kind(bool b_is_nk) { return b_is_nk ? Derived::kColumnSumsNK : Derived::kColumnSumsKN; }
+
+void *derived_lookup(const DerivedKey &key) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
-  auto it = g_padded_weights.find(PaddedKey{reinterpret_cast<uintptr_t>(ptr), k, n});
-  return it == g_padded_weights.end() ? nullptr : it->second;
+  auto it = g_derived.find(key);
+  return it == g_derived.end() ? nullptr : it->second;
 }
 // Two threads may have derived the same thing at once: the first one's stays (the other thread may
 // already be launching with it), the later one is given back.  Returns what the store holds.
-void *derived_insert(const void *ptr, int64_t k, int64_t n, void *data) {
+void *derived_insert(const DerivedKey &key, void *data) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
-  void *&slot = g_padded_weights[PaddedKey{reinterpret_cast<uintptr_t>(ptr), k, n}];
+  void *&slot = g_derived[key];
   if (slot) cudaFree(data);
   else slot = data;
   return slot;
 }
+// Drops what was derived from weights that start in [begin, end).  Call with g_const_mutex held.
+void drop_derived(uintptr_t begin, uintptr_t end) {
+  for (auto it = g_derived.lower_bound(DerivedKey{begin, INT64_MIN, INT64_MIN, Derived::kRepitched});
+       it != g_derived.end() && it->first.ptr < end;) {
+    cudaFree(it->second);
+    it = g_derived.erase(it);
+  }
+}
 }  // namespace
 
 const __half *padded_weight_lookup(const void *ptr, int64_t k, int64_t n) {
-  return static_cast<const __half *>(derived_lookup(ptr, k, n));
+  return static_cast<const __half *>(derived_lookup(derived_key(ptr, k, n, Derived::kRepitched)));
 }
 const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy) {
-  return static_cast<const __half *>(derived_insert(ptr, k, n, copy));
+  return static_cast<const __half *>(derived_insert(derived_key(ptr, k, n, Derived::kRepitched), copy));
 }
-const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n) {
-  return static_cast<const float *>(derived_lookup(ptr, k, -n));
+const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk) {
+  return static_cast<const float *>(derived_lookup(derived_key(ptr, k, n, column_sums_kind(b_is_nk))));
 }
-const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, float *sums) {
-  return static_cast<const float *>(derived_insert(ptr, k, -n, sums));
+const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, float *sums) {
+  return static_cast<const float *>(derived_insert(derived_key(ptr, k, n, column_sums_kind(b_is_nk)), sums));
 }
 
 void declare_constant_range(const void *ptr, size_t bytes) {
@@ -196,11 +212,7 @@ void declare_constant_range(const void *ptr, size_t bytes) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
   // A (re)declaration says "constant from now on": whatever was derived from an earlier content
   // of these addresses (re-pitched copies, column sums) is stale.
-  for (auto it = g_padded_weights.lower_bound(PaddedKey{b, INT64_MIN, INT64_MIN});
-       it != g_padded_weights.end() && it->first.ptr < b + bytes;) {
-    cudaFree(it->second);
-    it = g_padded_weights.erase(it);
-  }
+  drop_derived(b, b + bytes);
   g_const_ranges[b] = b + bytes;
 }
 
@@ -210,12 +222,7 @@ void forget_constant_range(const void *ptr) {
   auto range = g_const_ranges.find(b);
   const uintptr_t e = range == g_const_ranges.end() ? b + 1 : range->second;
   if (range != g_const_ranges.end()) g_const_ranges.erase(range);
-  // re-pitched copies of weights inside the withdrawn range go with it
-  for (auto it = g_padded_weights.lower_bound(PaddedKey{b, INT64_MIN, INT64_MIN});
-       it != g_padded_weights.end() && it->first.ptr < e;) {
-    cudaFree(it->second);
-    it = g_padded_weights.erase(it);
-  }
+  drop_derived(b, e);  // what was derived from weights inside the withdrawn range goes with it
 }
 
 bool is_constant_range(const void *ptr, size_t bytes) {

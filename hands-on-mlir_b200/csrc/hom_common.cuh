@@ -86,9 +86,10 @@ bool is_constant_range(const void *ptr, size_t bytes);
 const __half *padded_weight_lookup(const void *ptr, int64_t k, int64_t n);
 const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy);
 // The same store for the fp32 column sums of a declared weight (N floats; the LayerNorm-on-A
-// forms of the GEMM epilogue need them): computed once, dropped with the declaration.
-const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n);
-const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, float *sums);
+// forms of the GEMM epilogue need them), one entry per layout the buffer is read in: computed
+// once, dropped with the declaration.
+const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk);
+const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, float *sums);
 // Programmatic dependent launch is on unless HOM_DISABLE_PDL is set (diagnostics).
 bool pdl_enabled();
 // Host-mapped status word that device code writes on a bounded-wait expiry (device pointer).

@@ -440,7 +440,7 @@ float *col_sum_scratch() {
 const float *column_sums(const char *name, const hom::gemm::Problem &pb, cudaStream_t stream) {
   bool keep = pb.b_const;
   if (keep) {
-    if (const float *sums = hom::weight_colsum_lookup(pb.B, pb.K, pb.N)) return sums;
+    if (const float *sums = hom::weight_colsum_lookup(pb.B, pb.K, pb.N, pb.b_is_nk)) return sums;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
       cudaGetLastError();
@@ -472,7 +472,7 @@ const float *column_sums(const char *name, const hom::gemm::Problem &pb, cudaStr
       cudaFree(fresh);
       return nullptr;
     }
-    return hom::weight_colsum_insert(pb.B, pb.K, pb.N, fresh);
+    return hom::weight_colsum_insert(pb.B, pb.K, pb.N, pb.b_is_nk, fresh);
   }
   return fresh;
 }

@@ -69,3 +69,41 @@ def test_column_sums_of_a_weight_first_seen_under_capture(hom, cuda):
     finally:
         hom.use_torch_stream()
         hom.forget_weights(tB)
+
+
+def _partials(x):
+    """{sum, sum of squares} of every row per 64-column group, [groups, rows, 2] fp32."""
+    g = x.astype(np.float32).reshape(x.shape[0], -1, 64)
+    return np.ascontiguousarray(np.stack([g.sum(-1), (g * g).sum(-1)], axis=-1).transpose(1, 0, 2))
+
+
+@pytest.mark.parametrize("first", ["kn", "nk"])
+def test_a_square_weight_read_in_both_layouts(hom, cuda, first):
+    """One declared buffer taken as [K, N] by one entry point and as [N, K] by another: each gets the
+    sums of its own layout, whichever of them came first."""
+    import torch
+
+    m, n = 64, 128
+    A, B, rstd, shift, want_kn = _case(m, n, n, 7)
+    a, b = A[0].astype(np.float64), B[0].astype(np.float64)
+    mean, var = a.mean(-1, keepdims=True), a.var(-1, keepdims=True)
+    want_nk = (((a - mean) / np.sqrt(var + 1e-12)) @ b.T)[None]
+    tA, tB, tV, tM, tS = (to_dev(x, cuda) for x in (A, B, rstd, shift, _partials(A[0])))
+    tD = torch.zeros((1, m, n), dtype=torch.float16, device=cuda)
+
+    def kn():
+        hom.cutlassLayernormGemmF16(tA, tB, None, tD, tV, tM)
+        hom.synchronize()
+        assert_close_f16(tD.cpu().numpy(), want_kn, "[K, N]")
+
+    def nk():
+        hom.homGemmDeferredLayernormF16(tA, tS, tB, None, None, tD, None, weights_nk=True)
+        hom.synchronize()
+        assert_close_f16(tD.cpu().numpy(), want_nk, "[N, K]")
+
+    hom.declare_weights(tB)
+    try:
+        for call in (kn, nk, kn) if first == "kn" else (nk, kn, nk):
+            call()
+    finally:
+        hom.forget_weights(tB)
