@@ -151,6 +151,65 @@ bool split_workspace(size_t slot_floats, size_t blocks, cudaStream_t stream, Spl
 }
 
 namespace {
+// Device memory nobody uses any more, waiting for a cudaFree: the last owner can be a graph, whose
+// release callback may not call CUDA.  Never destroyed (such a callback may come during exit).
+struct FreeList {
+  std::mutex mu;
+  std::vector<void *> ptrs;
+};
+FreeList &free_list() {
+  static FreeList *list = new FreeList;
+  return *list;
+}
+void release_from_graph(void *ptr) {
+  FreeList &list = free_list();
+  std::lock_guard<std::mutex> lock(list.mu);
+  list.ptrs.push_back(ptr);
+}
+void free_released_memory() {
+  FreeList &list = free_list();
+  std::vector<void *> ptrs;
+  {
+    std::lock_guard<std::mutex> lock(list.mu);
+    ptrs.swap(list.ptrs);
+  }
+  for (void *ptr : ptrs) cudaFree(ptr);
+}
+}  // namespace
+
+bool is_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st == cudaStreamCaptureStatusActive;
+  cudaGetLastError();  // the legacy stream while another one is captured: the launch will say so
+  return false;
+}
+
+void *graph_owned_memory(size_t bytes, cudaStream_t stream, const char *what) {
+  CaptureSafeCalls safe;
+  free_released_memory();
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (!check_cuda(cudaStreamGetCaptureInfo_v2(stream, &st, &id, &graph), what)) return nullptr;
+  if (st != cudaStreamCaptureStatusActive) {
+    set_error(HOM_ERR_CUDA, "%s: the stream is not being captured", what);
+    return nullptr;
+  }
+  void *ptr = nullptr;
+  if (!check_cuda(cudaMalloc(&ptr, bytes), what)) return nullptr;
+  cudaUserObject_t owner = nullptr;
+  if (!check_cuda(cudaUserObjectCreate(&owner, ptr, release_from_graph, 1, cudaUserObjectNoDestructorSync), what)) {
+    cudaFree(ptr);
+    return nullptr;
+  }
+  if (!check_cuda(cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove), what)) {
+    cudaUserObjectRelease(owner, 1);  // queues ptr
+    return nullptr;
+  }
+  return ptr;
+}
+
+namespace {
 enum class Derived : int { kRepitched, kColumnSumsKN, kColumnSumsNK };
 struct DerivedKey {
   uintptr_t ptr;
@@ -208,6 +267,7 @@ const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_
 
 void declare_constant_range(const void *ptr, size_t bytes) {
   if (!ptr || bytes == 0) return;
+  free_released_memory();
   const uintptr_t b = reinterpret_cast<uintptr_t>(ptr);
   std::lock_guard<std::mutex> lock(g_const_mutex);
   // A (re)declaration says "constant from now on": whatever was derived from an earlier content
@@ -217,6 +277,7 @@ void declare_constant_range(const void *ptr, size_t bytes) {
 }
 
 void forget_constant_range(const void *ptr) {
+  free_released_memory();
   std::lock_guard<std::mutex> lock(g_const_mutex);
   const uintptr_t b = reinterpret_cast<uintptr_t>(ptr);
   auto range = g_const_ranges.find(b);

@@ -90,6 +90,23 @@ const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half
 // once, dropped with the declaration.
 const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk);
 const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, float *sums);
+// For the lifetime of the object this thread may allocate and free although some stream is being
+// captured (cudaMalloc and cudaFree are not stream operations; the default capture mode refuses
+// them to guard against programs that mean them to be part of the graph).
+class CaptureSafeCalls {
+ public:
+  CaptureSafeCalls() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  ~CaptureSafeCalls() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  CaptureSafeCalls(const CaptureSafeCalls &) = delete;
+  CaptureSafeCalls &operator=(const CaptureSafeCalls &) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+bool is_capturing(cudaStream_t stream);
+// Device memory for one captured call: it lives as long as the graph (and what is instantiated
+// from it), so replays of graphs on any streams do not share it.  Null (error recorded) on failure.
+void *graph_owned_memory(size_t bytes, cudaStream_t stream, const char *what);
 // Programmatic dependent launch is on unless HOM_DISABLE_PDL is set (diagnostics).
 bool pdl_enabled();
 // Host-mapped status word that device code writes on a bounded-wait expiry (device pointer).

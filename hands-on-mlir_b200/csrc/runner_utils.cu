@@ -435,30 +435,30 @@ float *col_sum_scratch() {
 
 // The column sums of pb.B (fp32).  Those of a declared weight are computed once and kept until the
 // declaration is withdrawn or renewed, those of any other B on every call.  While the stream is
-// being captured nothing can be allocated or waited for, so sums that are not there yet are
-// computed into the scratch as part of the graph.  Null (error recorded) on failure.
-const float *column_sums(const char *name, const hom::gemm::Problem &pb, cudaStream_t stream) {
-  bool keep = pb.b_const;
-  if (keep) {
+// being captured nothing can be waited for, so sums that are not there yet are computed as part of
+// the graph, into memory of its own.  `kept_in_graphs` false: the sums of a captured call are
+// always part of the graph, which then follows weights that are rewritten between replays and
+// holds no address that a new declaration gives back.  Null (error recorded) on failure.
+const float *column_sums(const char *name, const hom::gemm::Problem &pb, bool kept_in_graphs, cudaStream_t stream) {
+  const bool capturing = hom::is_capturing(stream);
+  if (pb.b_const && (!capturing || kept_in_graphs))
     if (const float *sums = hom::weight_colsum_lookup(pb.B, pb.K, pb.N, pb.b_is_nk)) return sums;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      keep = false;
-    }
+  const size_t bytes = static_cast<size_t>(pb.N) * sizeof(float);
+  const bool keep = pb.b_const && !capturing;
+  if (!keep && pb.N > kColSumCapacity) {
+    set_error(HOM_ERR_UNSUPPORTED, "%s: N = %lld exceeds the %lld-column scratch", name,
+              static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
+    return nullptr;
   }
   float *fresh = nullptr;
-  if (keep) {
+  if (capturing) {
+    fresh = static_cast<float *>(hom::graph_owned_memory(bytes, stream, "column sums of a captured call"));
+    if (!fresh) return nullptr;
+  } else if (keep) {
     void *ptr = nullptr;
-    if (!hom::check_cuda(cudaMalloc(&ptr, static_cast<size_t>(pb.N) * sizeof(float)), "cudaMalloc(column sums)"))
-      return nullptr;
+    if (!hom::check_cuda(cudaMalloc(&ptr, bytes), "cudaMalloc(column sums)")) return nullptr;
     fresh = static_cast<float *>(ptr);
   } else {
-    if (pb.N > kColSumCapacity) {
-      set_error(HOM_ERR_UNSUPPORTED, "%s: N = %lld exceeds the %lld-column scratch", name,
-                static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
-      return nullptr;
-    }
     fresh = col_sum_scratch();
     if (!fresh) return nullptr;
   }
@@ -695,7 +695,7 @@ void cutlassLayernormGemmF16(int64_t rankA, void *dstA, int64_t rankB, void *dst
   }
   pb.row_scale = var;
   pb.row_shift = mean;
-  pb.col_sum = column_sums("cutlassLayernormGemmF16", pb, hom::current_stream());
+  pb.col_sum = column_sums("cutlassLayernormGemmF16", pb, /*kept_in_graphs=*/false, hom::current_stream());
   if (!pb.col_sum) return;
   hom::gemm::run(pb, 0, hom::current_stream());
 }
@@ -846,7 +846,7 @@ void homGemmDeferredLayernormF16(int64_t rankA, void *dstA, int64_t rankStatsA, 
   cudaStream_t stream = hom::current_stream();
   if (stats_a) {
     // LayerNorm(A).B = rstd * (A.B) - mean * rstd * colsum(B)
-    const float *sums = column_sums(name, pb, stream);
+    const float *sums = column_sums(name, pb, /*kept_in_graphs=*/true, stream);
     if (!sums) return;
     pb.col_sum = sums;
     pb.a_partials = stats_a;

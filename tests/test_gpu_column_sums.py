@@ -107,3 +107,64 @@ def test_a_square_weight_read_in_both_layouts(hom, cuda, first):
             call()
     finally:
         hom.forget_weights(tB)
+
+
+def test_a_captured_call_follows_a_rewritten_weight(hom, cuda):
+    """A graph captured when the weight's sums were already kept: rewriting the weight and declaring
+    it again (which gives the kept sums back) leaves the graph valid, and it follows the contents."""
+    import torch
+
+    A, B, rstd, shift, want = _case(64, 256, 128, 11)
+    tA, tB, tV, tM = (to_dev(x, cuda) for x in (A, B, rstd, shift))
+    tD = torch.zeros((1, 64, 256), dtype=torch.float16, device=cuda)
+    hom.declare_weights(tB)
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    try:
+        hom.cutlassLayernormGemmF16(tA, tB, None, tD, tV, tM)
+        hom.synchronize()
+        hom.set_stream(stream.cuda_stream)
+        with torch.cuda.graph(graph, stream=stream):
+            hom.cutlassLayernormGemmF16(tA, tB, None, tD, tV, tM)
+        for factor in (1, -1, 0.5):
+            tB.copy_(torch.from_numpy(B)).mul_(factor)
+            hom.declare_weights(tB)
+            tD.zero_()
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert_close_f16(tD.cpu().numpy(), want.astype(np.float64) * factor, f"weights x {factor}")
+    finally:
+        hom.use_torch_stream()
+        hom.forget_weights(tB)
+
+
+def test_captured_calls_do_not_share_their_sums(hom, cuda):
+    """Two graphs captured on one stream, with different weights, replayed on two streams at once;
+    then both destroyed and captured again."""
+    import torch
+
+    cases = [_case(256, 512, 512, seed) for seed in (21, 22)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    dev = [[to_dev(x, cuda) for x in c[:4]] + [torch.zeros((1, 256, 512), dtype=torch.float16, device=cuda)]
+           for c in cases]
+    torch.cuda.synchronize()
+    try:
+        hom.set_stream(streams[0].cuda_stream)
+        for _ in range(3):
+            graphs = [torch.cuda.CUDAGraph() for _ in cases]
+            for graph, (tA, tB, tV, tM, tD) in zip(graphs, dev):
+                with torch.cuda.graph(graph, stream=streams[0]):
+                    for _ in range(8):
+                        hom.cutlassLayernormGemmF16(tA, tB, None, tD, tV, tM)
+            for _ in range(20):
+                for graph, stream in zip(graphs, streams):
+                    with torch.cuda.stream(stream):
+                        graph.replay()
+            torch.cuda.synchronize()
+            for case, d in zip(cases, dev):
+                assert_close_f16(d[4].cpu().numpy(), case[4], "replayed on two streams")
+                d[4].zero_()
+            del graphs
+    finally:
+        hom.use_torch_stream()
