@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -161,11 +162,6 @@ FreeList &free_list() {
   static FreeList *list = new FreeList;
   return *list;
 }
-void release_from_graph(void *ptr) {
-  FreeList &list = free_list();
-  std::lock_guard<std::mutex> lock(list.mu);
-  list.ptrs.push_back(ptr);
-}
 void free_released_memory() {
   FreeList &list = free_list();
   std::vector<void *> ptrs;
@@ -177,6 +173,20 @@ void free_released_memory() {
 }
 }  // namespace
 
+DeviceBuffer::~DeviceBuffer() {
+  FreeList &list = free_list();
+  std::lock_guard<std::mutex> lock(list.mu);
+  list.ptrs.push_back(data_);
+}
+
+SharedBuffer device_buffer(size_t bytes, const char *what) {
+  CaptureSafeCalls safe;
+  free_released_memory();
+  void *ptr = nullptr;
+  if (!check_cuda(cudaMalloc(&ptr, bytes), what)) return nullptr;
+  return std::make_shared<DeviceBuffer>(ptr);
+}
+
 bool is_capturing(cudaStream_t stream) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st == cudaStreamCaptureStatusActive;
@@ -184,29 +194,26 @@ bool is_capturing(cudaStream_t stream) {
   return false;
 }
 
-void *graph_owned_memory(size_t bytes, cudaStream_t stream, const char *what) {
-  CaptureSafeCalls safe;
-  free_released_memory();
+bool keep_for_graph(const SharedBuffer &buffer, cudaStream_t stream) {
+  const char *what = "device memory of a captured call";
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
   cudaGraph_t graph = nullptr;
-  if (!check_cuda(cudaStreamGetCaptureInfo_v2(stream, &st, &id, &graph), what)) return nullptr;
-  if (st != cudaStreamCaptureStatusActive) {
-    set_error(HOM_ERR_CUDA, "%s: the stream is not being captured", what);
-    return nullptr;
-  }
-  void *ptr = nullptr;
-  if (!check_cuda(cudaMalloc(&ptr, bytes), what)) return nullptr;
+  if (!check_cuda(cudaStreamGetCaptureInfo_v2(stream, &st, &id, &graph), what)) return false;
+  if (st != cudaStreamCaptureStatusActive) return true;
+  auto *share = new SharedBuffer(buffer);
   cudaUserObject_t owner = nullptr;
-  if (!check_cuda(cudaUserObjectCreate(&owner, ptr, release_from_graph, 1, cudaUserObjectNoDestructorSync), what)) {
-    cudaFree(ptr);
-    return nullptr;
+  if (!check_cuda(cudaUserObjectCreate(&owner, share, [](void *p) { delete static_cast<SharedBuffer *>(p); }, 1,
+                                       cudaUserObjectNoDestructorSync),
+                  what)) {
+    delete share;
+    return false;
   }
   if (!check_cuda(cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove), what)) {
-    cudaUserObjectRelease(owner, 1);  // queues ptr
-    return nullptr;
+    cudaUserObjectRelease(owner, 1);
+    return false;
   }
-  return ptr;
+  return true;
 }
 
 namespace {
@@ -221,69 +228,69 @@ struct DerivedKey {
     return std::tie(ptr, k, n, kind) < std::tie(o.ptr, o.k, o.n, o.kind);
   }
 };
-std::map<DerivedKey, void *> g_derived;  // guarded by g_const_mutex
+std::map<DerivedKey, SharedBuffer> g_derived;  // guarded by g_const_mutex
 
 DerivedKey derived_key(const void *ptr, int64_t k, int64_t n, Derived kind) {
   return DerivedKey{reinterpret_cast<uintptr_t>(ptr), k, n, kind};
 }
 Derived column_sums_kind(bool b_is_nk) { return b_is_nk ? Derived::kColumnSumsNK : Derived::kColumnSumsKN; }
 
-void *derived_lookup(const DerivedKey &key) {
+SharedBuffer derived_lookup(const DerivedKey &key) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
   auto it = g_derived.find(key);
   return it == g_derived.end() ? nullptr : it->second;
 }
-// Two threads may have derived the same thing at once: the first one's stays (the other thread may
-// already be launching with it), the later one is given back.  Returns what the store holds.
-void *derived_insert(const DerivedKey &key, void *data) {
+// Two threads may have derived the same thing at once: the first one's stays.  Returns what the
+// store holds.
+SharedBuffer derived_insert(const DerivedKey &key, const SharedBuffer &data) {
   std::lock_guard<std::mutex> lock(g_const_mutex);
-  void *&slot = g_derived[key];
-  if (slot) cudaFree(data);
-  else slot = data;
-  return slot;
+  return g_derived.emplace(key, data).first->second;
 }
-// Drops what was derived from weights that start in [begin, end).  Call with g_const_mutex held.
+// Drops what was derived from weights that start in [begin, end).  Call with g_const_mutex held;
+// the memory waits in the free list for its last user.
 void drop_derived(uintptr_t begin, uintptr_t end) {
   for (auto it = g_derived.lower_bound(DerivedKey{begin, INT64_MIN, INT64_MIN, Derived::kRepitched});
-       it != g_derived.end() && it->first.ptr < end;) {
-    cudaFree(it->second);
+       it != g_derived.end() && it->first.ptr < end;)
     it = g_derived.erase(it);
-  }
 }
 }  // namespace
 
-const __half *padded_weight_lookup(const void *ptr, int64_t k, int64_t n) {
-  return static_cast<const __half *>(derived_lookup(derived_key(ptr, k, n, Derived::kRepitched)));
+SharedBuffer padded_weight_lookup(const void *ptr, int64_t k, int64_t n) {
+  return derived_lookup(derived_key(ptr, k, n, Derived::kRepitched));
 }
-const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy) {
-  return static_cast<const __half *>(derived_insert(derived_key(ptr, k, n, Derived::kRepitched), copy));
+SharedBuffer padded_weight_insert(const void *ptr, int64_t k, int64_t n, const SharedBuffer &copy) {
+  return derived_insert(derived_key(ptr, k, n, Derived::kRepitched), copy);
 }
-const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk) {
-  return static_cast<const float *>(derived_lookup(derived_key(ptr, k, n, column_sums_kind(b_is_nk))));
+SharedBuffer weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk) {
+  return derived_lookup(derived_key(ptr, k, n, column_sums_kind(b_is_nk)));
 }
-const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, float *sums) {
-  return static_cast<const float *>(derived_insert(derived_key(ptr, k, n, column_sums_kind(b_is_nk)), sums));
+SharedBuffer weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, const SharedBuffer &sums) {
+  return derived_insert(derived_key(ptr, k, n, column_sums_kind(b_is_nk)), sums);
 }
 
 void declare_constant_range(const void *ptr, size_t bytes) {
   if (!ptr || bytes == 0) return;
-  free_released_memory();
   const uintptr_t b = reinterpret_cast<uintptr_t>(ptr);
-  std::lock_guard<std::mutex> lock(g_const_mutex);
-  // A (re)declaration says "constant from now on": whatever was derived from an earlier content
-  // of these addresses (re-pitched copies, column sums) is stale.
-  drop_derived(b, b + bytes);
-  g_const_ranges[b] = b + bytes;
+  {
+    std::lock_guard<std::mutex> lock(g_const_mutex);
+    // A (re)declaration says "constant from now on": whatever was derived from an earlier content
+    // of these addresses (re-pitched copies, column sums) is stale.
+    drop_derived(b, b + bytes);
+    g_const_ranges[b] = b + bytes;
+  }
+  free_released_memory();
 }
 
 void forget_constant_range(const void *ptr) {
+  {
+    std::lock_guard<std::mutex> lock(g_const_mutex);
+    const uintptr_t b = reinterpret_cast<uintptr_t>(ptr);
+    auto range = g_const_ranges.find(b);
+    const uintptr_t e = range == g_const_ranges.end() ? b + 1 : range->second;
+    if (range != g_const_ranges.end()) g_const_ranges.erase(range);
+    drop_derived(b, e);  // what was derived from weights inside the withdrawn range goes with it
+  }
   free_released_memory();
-  std::lock_guard<std::mutex> lock(g_const_mutex);
-  const uintptr_t b = reinterpret_cast<uintptr_t>(ptr);
-  auto range = g_const_ranges.find(b);
-  const uintptr_t e = range == g_const_ranges.end() ? b + 1 : range->second;
-  if (range != g_const_ranges.end()) g_const_ranges.erase(range);
-  drop_derived(b, e);  // what was derived from weights inside the withdrawn range goes with it
 }
 
 bool is_constant_range(const void *ptr, size_t bytes) {

@@ -5,6 +5,8 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
+
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -78,18 +80,6 @@ cudaStream_t current_stream();
 void declare_constant_range(const void *ptr, size_t bytes);
 void forget_constant_range(const void *ptr);
 bool is_constant_range(const void *ptr, size_t bytes);
-// Library-owned copies of declared-constant [K, N] weights whose N is not a multiple of 8,
-// re-laid-out with an 8-element-aligned row pitch so that TMA can fetch them; keyed on the
-// original pointer and shape, dropped when the declaration is withdrawn.  lookup returns null
-// when there is none yet; insert takes ownership of a cudaMalloc'ed copy and
-// returns the one in the store (an earlier one if another thread was first).
-const __half *padded_weight_lookup(const void *ptr, int64_t k, int64_t n);
-const __half *padded_weight_insert(const void *ptr, int64_t k, int64_t n, __half *copy);
-// The same store for the fp32 column sums of a declared weight (N floats; the LayerNorm-on-A
-// forms of the GEMM epilogue need them), one entry per layout the buffer is read in: computed
-// once, dropped with the declaration.
-const float *weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk);
-const float *weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, float *sums);
 // For the lifetime of the object this thread may allocate and free although some stream is being
 // captured (cudaMalloc and cudaFree are not stream operations; the default capture mode refuses
 // them to guard against programs that mean them to be part of the graph).
@@ -104,9 +94,41 @@ class CaptureSafeCalls {
   cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
 };
 bool is_capturing(cudaStream_t stream);
-// Device memory for one captured call: it lives as long as the graph (and what is instantiated
-// from it), so replays of graphs on any streams do not share it.  Null (error recorded) on failure.
-void *graph_owned_memory(size_t bytes, cudaStream_t stream, const char *what);
+
+// Device memory that its users own together: the store of derived buffers below, a call that is
+// about to launch with it, and the graphs that were captured with its address.  When the last of
+// them is gone it is freed by the next call that allocates, declares or forgets.
+class DeviceBuffer {
+ public:
+  explicit DeviceBuffer(void *data) : data_(data) {}
+  ~DeviceBuffer();
+  DeviceBuffer(const DeviceBuffer &) = delete;
+  DeviceBuffer &operator=(const DeviceBuffer &) = delete;
+  template <typename T>
+  T *as() const { return static_cast<T *>(data_); }
+
+ private:
+  void *data_;
+};
+using SharedBuffer = std::shared_ptr<DeviceBuffer>;
+// Null (error recorded) on failure.
+SharedBuffer device_buffer(size_t bytes, const char *what);
+// When `stream` is being captured, makes the graph (and what is instantiated from it) an owner of
+// `buffer`; call it before launching with the buffer.  False (error recorded) on failure.
+bool keep_for_graph(const SharedBuffer &buffer, cudaStream_t stream);
+
+// Library-owned copies of declared-constant [K, N] weights whose N is not a multiple of 8,
+// re-laid-out with an 8-element-aligned row pitch so that TMA can fetch them; keyed on the
+// original pointer and shape, dropped when the declaration is withdrawn or renewed.  lookup returns
+// null when there is none yet; insert returns the one in the store (an earlier one if another
+// thread was first).
+SharedBuffer padded_weight_lookup(const void *ptr, int64_t k, int64_t n);
+SharedBuffer padded_weight_insert(const void *ptr, int64_t k, int64_t n, const SharedBuffer &copy);
+// The same store for the fp32 column sums of a declared weight (N floats; the LayerNorm-on-A
+// forms of the GEMM epilogue need them), one entry per layout the buffer is read in: computed
+// once, dropped with the declaration.
+SharedBuffer weight_colsum_lookup(const void *ptr, int64_t k, int64_t n, bool b_is_nk);
+SharedBuffer weight_colsum_insert(const void *ptr, int64_t k, int64_t n, bool b_is_nk, const SharedBuffer &sums);
 // Programmatic dependent launch is on unless HOM_DISABLE_PDL is set (diagnostics).
 bool pdl_enabled();
 // Host-mapped status word that device code writes on a bounded-wait expiry (device pointer).

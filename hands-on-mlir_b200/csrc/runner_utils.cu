@@ -354,48 +354,38 @@ bool gemm_prepare(const char *name, bool b_is_nk, int64_t rankA, void *dstA, int
 // aligned, so TMA cannot fetch it in place.  The GEMM runs on a copy whose row pitch is rounded
 // up to 8 elements: made once and kept for a declared constant (model weights), re-made on every
 // call into a grow-only scratch of the calling thread for any other B.
-bool repitch_unaligned_b(const char *name, hom::gemm::Problem *pb) {
+// `owner` keeps the copy alive until the caller has launched with it.
+bool repitch_unaligned_b(hom::gemm::Problem *pb, hom::SharedBuffer *owner) {
   const int64_t pitch = (pb->N + 7) / 8 * 8;
+  const size_t elems = static_cast<size_t>(pb->K) * pitch;
   cudaStream_t stream = hom::current_stream();
-  const __half *copy = pb->b_const ? hom::padded_weight_lookup(pb->B, pb->K, pb->N) : nullptr;
-  if (!copy) {
-    __half *fresh = nullptr;
-    if (pb->b_const) {
-      void *ptr = nullptr;
-      if (!hom::check_cuda(cudaMalloc(&ptr, static_cast<size_t>(pb->K) * pitch * 2), "cudaMalloc(re-pitched weights)"))
-        return false;
-      fresh = static_cast<__half *>(ptr);
-    } else {
-      thread_local __half *scratch = nullptr;
-      thread_local size_t scratch_elems = 0;
-      const size_t need = static_cast<size_t>(pb->K) * pitch;
-      if (scratch_elems < need) {
-        if (scratch) cudaFree(scratch);  // waits for the kernels that may still read it
-        scratch = nullptr;
-        scratch_elems = 0;
-        void *ptr = nullptr;
-        if (!hom::check_cuda(cudaMalloc(&ptr, need * 2), "cudaMalloc(re-pitched B)")) return false;
-        scratch = static_cast<__half *>(ptr);
-        scratch_elems = need;
-      }
-      fresh = scratch;
-    }
-    if (!hom::bw::repitch_rows_f16(pb->B, fresh, pb->K, pb->N, pitch, stream)) {
-      if (pb->b_const) cudaFree(fresh);
-      return false;
-    }
-    if (pb->b_const) {
+  const __half *copy = nullptr;
+  if (pb->b_const) {
+    *owner = hom::padded_weight_lookup(pb->B, pb->K, pb->N);
+    if (!*owner) {
+      hom::SharedBuffer fresh = hom::device_buffer(elems * 2, "cudaMalloc(re-pitched weights)");
+      if (!fresh || !hom::bw::repitch_rows_f16(pb->B, fresh->as<__half>(), pb->K, pb->N, pitch, stream)) return false;
       // other streams may use the cached copy next: make it complete before it becomes visible
-      if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(re-pitched weights)")) {
-        cudaFree(fresh);
-        return false;
-      }
-      copy = hom::padded_weight_insert(pb->B, pb->K, pb->N, fresh);
-    } else {
-      copy = fresh;
+      if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(re-pitched weights)")) return false;
+      *owner = hom::padded_weight_insert(pb->B, pb->K, pb->N, fresh);
     }
+    if (!hom::keep_for_graph(*owner, stream)) return false;
+    copy = (*owner)->as<__half>();
+  } else {
+    thread_local __half *scratch = nullptr;
+    thread_local size_t scratch_elems = 0;
+    if (scratch_elems < elems) {
+      if (scratch) cudaFree(scratch);  // waits for the kernels that may still read it
+      scratch = nullptr;
+      scratch_elems = 0;
+      void *ptr = nullptr;
+      if (!hom::check_cuda(cudaMalloc(&ptr, elems * 2), "cudaMalloc(re-pitched B)")) return false;
+      scratch = static_cast<__half *>(ptr);
+      scratch_elems = elems;
+    }
+    if (!hom::bw::repitch_rows_f16(pb->B, scratch, pb->K, pb->N, pitch, stream)) return false;
+    copy = scratch;
   }
-  (void)name;
   pb->B = copy;
   pb->ldb = pitch;
   return true;
@@ -410,7 +400,8 @@ void gemm_entry(const char *name, bool b_is_nk, int64_t rankA, void *dstA, int64
   if (!gemm_prepare(name, b_is_nk, rankA, dstA, rankB, dstB, rankC, dstC, rankD, dstD, activation,
                     alpha, beta, &pb, &empty, /*allow_unaligned_kn=*/true))
     return;
-  if (!b_is_nk && pb.N % 8 != 0 && !repitch_unaligned_b(name, &pb)) return;
+  hom::SharedBuffer copy_of_b;
+  if (!b_is_nk && pb.N % 8 != 0 && !repitch_unaligned_b(&pb, &copy_of_b)) return;
   pb.split_k = split_k;
   hom::gemm::run(pb, tile_row, hom::current_stream());
 }
@@ -437,44 +428,37 @@ float *col_sum_scratch() {
 // declaration is withdrawn or renewed, those of any other B on every call.  While the stream is
 // being captured nothing can be waited for, so sums that are not there yet are computed as part of
 // the graph, into memory of its own.  `kept_in_graphs` false: the sums of a captured call are
-// always part of the graph, which then follows weights that are rewritten between replays and
-// holds no address that a new declaration gives back.  Null (error recorded) on failure.
-const float *column_sums(const char *name, const hom::gemm::Problem &pb, bool kept_in_graphs, cudaStream_t stream) {
+// always part of the graph, which then follows weights that are rewritten between replays.
+// `owner` keeps the sums alive until the caller has launched with them.  Null (error recorded) on
+// failure.
+const float *column_sums(const char *name, const hom::gemm::Problem &pb, bool kept_in_graphs, cudaStream_t stream,
+                         hom::SharedBuffer *owner) {
   const bool capturing = hom::is_capturing(stream);
-  if (pb.b_const && (!capturing || kept_in_graphs))
-    if (const float *sums = hom::weight_colsum_lookup(pb.B, pb.K, pb.N, pb.b_is_nk)) return sums;
-  const size_t bytes = static_cast<size_t>(pb.N) * sizeof(float);
+  if (pb.b_const && (!capturing || kept_in_graphs)) {
+    *owner = hom::weight_colsum_lookup(pb.B, pb.K, pb.N, pb.b_is_nk);
+    if (*owner) return !capturing || hom::keep_for_graph(*owner, stream) ? (*owner)->as<float>() : nullptr;
+  }
   const bool keep = pb.b_const && !capturing;
   if (!keep && pb.N > kColSumCapacity) {
     set_error(HOM_ERR_UNSUPPORTED, "%s: N = %lld exceeds the %lld-column scratch", name,
               static_cast<long long>(pb.N), static_cast<long long>(kColSumCapacity));
     return nullptr;
   }
-  float *fresh = nullptr;
-  if (capturing) {
-    fresh = static_cast<float *>(hom::graph_owned_memory(bytes, stream, "column sums of a captured call"));
-    if (!fresh) return nullptr;
-  } else if (keep) {
-    void *ptr = nullptr;
-    if (!hom::check_cuda(cudaMalloc(&ptr, bytes), "cudaMalloc(column sums)")) return nullptr;
-    fresh = static_cast<float *>(ptr);
+  float *sums = nullptr;
+  if (keep || capturing) {
+    *owner = hom::device_buffer(static_cast<size_t>(pb.N) * sizeof(float), "cudaMalloc(column sums)");
+    if (!*owner || (capturing && !hom::keep_for_graph(*owner, stream))) return nullptr;
+    sums = (*owner)->as<float>();
   } else {
-    fresh = col_sum_scratch();
-    if (!fresh) return nullptr;
+    sums = col_sum_scratch();
+    if (!sums) return nullptr;
   }
-  if (!hom::bw::col_sum_f16(pb.B, fresh, pb.K, pb.N, pb.b_is_nk, stream)) {
-    if (keep) cudaFree(fresh);
-    return nullptr;
-  }
-  if (keep) {
-    // other streams may use the kept sums next: make them complete before they become visible
-    if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(column sums)")) {
-      cudaFree(fresh);
-      return nullptr;
-    }
-    return hom::weight_colsum_insert(pb.B, pb.K, pb.N, pb.b_is_nk, fresh);
-  }
-  return fresh;
+  if (!hom::bw::col_sum_f16(pb.B, sums, pb.K, pb.N, pb.b_is_nk, stream)) return nullptr;
+  if (!keep) return sums;
+  // other streams may use the kept sums next: make them complete before they become visible
+  if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(column sums)")) return nullptr;
+  *owner = hom::weight_colsum_insert(pb.B, pb.K, pb.N, pb.b_is_nk, *owner);
+  return (*owner)->as<float>();
 }
 
 // Var / Mean operands of the fused forms: rank-1 fp16 with at least `rows` entries.
@@ -695,7 +679,8 @@ void cutlassLayernormGemmF16(int64_t rankA, void *dstA, int64_t rankB, void *dst
   }
   pb.row_scale = var;
   pb.row_shift = mean;
-  pb.col_sum = column_sums("cutlassLayernormGemmF16", pb, /*kept_in_graphs=*/false, hom::current_stream());
+  hom::SharedBuffer sums;
+  pb.col_sum = column_sums("cutlassLayernormGemmF16", pb, /*kept_in_graphs=*/false, hom::current_stream(), &sums);
   if (!pb.col_sum) return;
   hom::gemm::run(pb, 0, hom::current_stream());
 }
@@ -844,11 +829,11 @@ void homGemmDeferredLayernormF16(int64_t rankA, void *dstA, int64_t rankStatsA, 
     return;
   }
   cudaStream_t stream = hom::current_stream();
+  hom::SharedBuffer sums;
   if (stats_a) {
     // LayerNorm(A).B = rstd * (A.B) - mean * rstd * colsum(B)
-    const float *sums = column_sums(name, pb, /*kept_in_graphs=*/true, stream);
-    if (!sums) return;
-    pb.col_sum = sums;
+    pb.col_sum = column_sums(name, pb, /*kept_in_graphs=*/true, stream, &sums);
+    if (!pb.col_sum) return;
     pb.a_partials = stats_a;
     pb.a_groups = static_cast<int>(ga);
   }

@@ -1,6 +1,8 @@
 """LayerNorm-on-A GEMM: the column sums of B it needs, for shapes at the edges of the column-sum
 kernel (fewer columns than a block, a column tail, fewer and more rows than its warps), for weights
 that are declared (sums kept), not declared (computed on every call) and seen first under capture."""
+import time
+
 import numpy as np
 import pytest
 
@@ -168,3 +170,62 @@ def test_captured_calls_do_not_share_their_sums(hom, cuda):
             del graphs
     finally:
         hom.use_torch_stream()
+
+
+def test_a_graph_keeps_what_was_derived_from_its_weights(hom, cuda):
+    """What a graph was captured with (kept column sums, the re-pitched copy of an odd-N weight) stays
+    until the graph is gone, although the weights have been declared again in between."""
+    import torch
+
+    m, k, n = 64, 2048, 8196  # the copy of the second weight: 33.6 MB
+    A, B, _, _, _ = _case(m, 256, k, 31)
+    a, b = A[0].astype(np.float64), B[0].astype(np.float64)
+    mean, var = a.mean(-1, keepdims=True), a.var(-1, keepdims=True)
+    want = (((a - mean) / np.sqrt(var + 1e-12)) @ b)[None]
+    V = np.random.default_rng(32).normal(0, 0.02, (1, k, n)).astype(np.float16)
+    rows = torch.from_numpy(A).to(cuda)
+    tS, tB, tV = (to_dev(x, cuda) for x in (_partials(A[0]), B, V))
+    tD = torch.zeros((1, m, 256), dtype=torch.float16, device=cuda)
+    tL = torch.zeros((1, m, n), dtype=torch.float16, device=cuda)
+    want_l = a @ V[0].astype(np.float64)
+
+    def call():
+        hom.homGemmDeferredLayernormF16(rows, tS, tB, None, None, tD, None)
+        hom.cutlassGemmF16(rows, tV, None, tL)
+
+    def free_memory():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    for t in (tB, tV):
+        hom.declare_weights(t)
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    try:
+        call()
+        hom.synchronize()
+        hom.set_stream(stream.cuda_stream)
+        with torch.cuda.graph(graph, stream=stream):
+            call()
+        before = free_memory()
+        for t in (tB, tV):
+            hom.declare_weights(t)
+        assert free_memory() - before < 16 << 20, "the copy that the graph reads was freed"
+        tD.zero_()
+        tL.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_close_f16(tD.cpu().numpy(), want, "kept sums")
+        assert_close_f16(tL.cpu().numpy()[0], want_l, "re-pitched copy")
+        before = free_memory()
+        del graph
+        for _ in range(100):  # CUDA reports the end of a graph from a thread of its own
+            hom.declare_weights(tV)
+            if free_memory() - before >= 32 << 20:
+                break
+            time.sleep(0.05)
+        assert free_memory() - before >= 32 << 20, "the copy outlived the graph"
+    finally:
+        hom.use_torch_stream()
+        for t in (tB, tV):
+            hom.forget_weights(t)
