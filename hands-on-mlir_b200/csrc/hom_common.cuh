@@ -138,8 +138,9 @@ int *device_status_word();
 int *device_status_word_if_ready();
 int sm_count();
 
-// Library-owned split-K scratch of the calling host thread for (current device, `stream`):
-// `slot_floats` fp32 values of partial accumulators and `blocks` int counters that are zero
+// Library-owned scratch of the calling host thread for (current device, `stream`): `slot_floats`
+// fp32 values (partial accumulators of a split K; in GEMMs that are never split, row statistics or
+// column sums) and `blocks` int counters that are zero
 // whenever no GEMM is in flight.  Grow-only, allocated on first use (the reference keeps
 // grow-only static device scratch for its split-K semaphores too,
 // include/NVGPUKernels/Utils.h:179-224); growing it, or re-zeroing the counters after a kernel

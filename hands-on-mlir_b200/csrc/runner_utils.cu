@@ -406,26 +406,13 @@ void gemm_entry(const char *name, bool b_is_nk, int64_t rankA, void *dstA, int64
   hom::gemm::run(pb, tile_row, hom::current_stream());
 }
 
-// Library-owned scratch for the column sums of B that the LayerNorm-on-A GEMM needs: one
-// fixed buffer per device, allocated on first use (the reference keeps grow-only static device
-// scratch for the same kind of purpose, include/NVGPUKernels/Utils.h:179-224).
+// Widest B whose column sums are computed on every call (a bound on the scratch they need).
 constexpr int64_t kColSumCapacity = 65536;
-float *col_sum_scratch() {
-  static float *bufs[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!bufs[dev]) {
-    void *ptr = nullptr;
-    if (!hom::check_cuda(cudaMalloc(&ptr, kColSumCapacity * sizeof(float)), "cudaMalloc(column sums)"))
-      return nullptr;
-    bufs[dev] = static_cast<float *>(ptr);
-  }
-  return bufs[dev];
-}
 
 // The column sums of pb.B (fp32).  Those of a declared weight are computed once and kept until the
-// declaration is withdrawn or renewed, those of any other B on every call.  While the stream is
+// declaration is withdrawn or renewed, those of any other B on every call into the workspace of
+// this thread and stream (LayerNorm forms never split K, so the GEMM leaves it alone, and the next
+// call on the stream writes it after this one has finished).  While the stream is
 // being captured nothing can be waited for, so sums that are not there yet are computed as part of
 // the graph, into memory of its own.  `kept_in_graphs` false: the sums of a captured call are
 // always part of the graph, which then follows weights that are rewritten between replays.
@@ -450,8 +437,9 @@ const float *column_sums(const char *name, const hom::gemm::Problem &pb, bool ke
     if (!*owner || (capturing && !hom::keep_for_graph(*owner, stream))) return nullptr;
     sums = (*owner)->as<float>();
   } else {
-    sums = col_sum_scratch();
-    if (!sums) return nullptr;
+    hom::SplitWorkspace ws;
+    if (!hom::split_workspace(static_cast<size_t>(pb.N), 0, stream, &ws)) return nullptr;
+    sums = ws.slots;
   }
   if (!hom::bw::col_sum_f16(pb.B, sums, pb.K, pb.N, pb.b_is_nk, stream)) return nullptr;
   if (!keep) return sums;

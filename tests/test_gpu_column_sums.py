@@ -229,3 +229,36 @@ def test_a_graph_keeps_what_was_derived_from_its_weights(hom, cuda):
         hom.use_torch_stream()
         for t in (tB, tV):
             hom.forget_weights(t)
+
+
+def test_calls_on_two_streams_do_not_share_their_sums(hom, cuda):
+    """Weights that are not declared, one per stream, calls on the two streams interleaved."""
+    import torch
+
+    cases = [_case(64, 2048, 2048, seed) for seed in (41, 42)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    dev = [[to_dev(x, cuda) for x in c[:4]] + [torch.zeros((1, 64, 2048), dtype=torch.float16, device=cuda)
+                                               for _ in range(40)] for c in cases]
+
+    def call(i):
+        for stream, d in zip(streams, dev):
+            hom.set_stream(stream.cuda_stream)
+            hom.cutlassLayernormGemmF16(d[0], d[1], None, d[4 + i], d[2], d[3])
+
+    try:
+        call(0)
+        torch.cuda.synchronize()
+        gate = torch.cuda.Event()
+        torch.cuda._sleep(50_000_000)  # both queues fill behind this, then run at the same time
+        gate.record()
+        for stream in streams:
+            stream.wait_event(gate)
+        for i in range(40):
+            call(i)
+        torch.cuda.synchronize()
+    finally:
+        hom.use_torch_stream()
+    for case, d in zip(cases, dev):
+        assert_close_f16(d[4].cpu().numpy(), case[4], "first call")
+        for tD in d[5:]:
+            assert torch.equal(tD, d[4])
