@@ -120,6 +120,7 @@ bool split_workspace(size_t slot_floats, size_t blocks, cudaStream_t stream, Spl
     b.slots = nullptr;
     b.slot_floats = 0;
     void *ptr = nullptr;
+    CaptureSafeCalls safe;
     if (!check_cuda(cudaMalloc(&ptr, want * sizeof(float)), "cudaMalloc(split-K partials)")) return false;
     b.slots = static_cast<float *>(ptr);
     b.slot_floats = want;
@@ -192,6 +193,11 @@ bool is_capturing(cudaStream_t stream) {
   if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st == cudaStreamCaptureStatusActive;
   cudaGetLastError();  // the legacy stream while another one is captured: the launch will say so
   return false;
+}
+
+bool complete_before_sharing(cudaStream_t stream, const char *what) {
+  CaptureSafeCalls safe;
+  return check_cuda(cudaStreamSynchronize(stream), what);
 }
 
 bool keep_for_graph(const SharedBuffer &buffer, cudaStream_t stream) {

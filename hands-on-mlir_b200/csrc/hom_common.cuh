@@ -80,9 +80,9 @@ cudaStream_t current_stream();
 void declare_constant_range(const void *ptr, size_t bytes);
 void forget_constant_range(const void *ptr);
 bool is_constant_range(const void *ptr, size_t bytes);
-// For the lifetime of the object this thread may allocate and free although some stream is being
-// captured (cudaMalloc and cudaFree are not stream operations; the default capture mode refuses
-// them to guard against programs that mean them to be part of the graph).
+// For the lifetime of the object this thread may allocate, free and wait for a stream although some
+// other stream is being captured (the default capture mode refuses that, and breaks the capture, to
+// guard against programs that mean it to be part of the graph).
 class CaptureSafeCalls {
  public:
   CaptureSafeCalls() { cudaThreadExchangeStreamCaptureMode(&mode_); }
@@ -113,6 +113,8 @@ class DeviceBuffer {
 using SharedBuffer = std::shared_ptr<DeviceBuffer>;
 // Null (error recorded) on failure.
 SharedBuffer device_buffer(size_t bytes, const char *what);
+// Waits for `stream`, so that what it computed into a buffer may be read from any other stream.
+bool complete_before_sharing(cudaStream_t stream, const char *what);
 // When `stream` is being captured, makes the graph (and what is instantiated from it) an owner of
 // `buffer`; call it before launching with the buffer.  False (error recorded) on failure.
 bool keep_for_graph(const SharedBuffer &buffer, cudaStream_t stream);

@@ -366,7 +366,7 @@ bool repitch_unaligned_b(hom::gemm::Problem *pb, hom::SharedBuffer *owner) {
       hom::SharedBuffer fresh = hom::device_buffer(elems * 2, "cudaMalloc(re-pitched weights)");
       if (!fresh || !hom::bw::repitch_rows_f16(pb->B, fresh->as<__half>(), pb->K, pb->N, pitch, stream)) return false;
       // other streams may use the cached copy next: make it complete before it becomes visible
-      if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(re-pitched weights)")) return false;
+      if (!hom::complete_before_sharing(stream, "cudaStreamSynchronize(re-pitched weights)")) return false;
       *owner = hom::padded_weight_insert(pb->B, pb->K, pb->N, fresh);
     }
     if (!hom::keep_for_graph(*owner, stream)) return false;
@@ -444,7 +444,7 @@ const float *column_sums(const char *name, const hom::gemm::Problem &pb, bool ke
   if (!hom::bw::col_sum_f16(pb.B, sums, pb.K, pb.N, pb.b_is_nk, stream)) return nullptr;
   if (!keep) return sums;
   // other streams may use the kept sums next: make them complete before they become visible
-  if (!hom::check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(column sums)")) return nullptr;
+  if (!hom::complete_before_sharing(stream, "cudaStreamSynchronize(column sums)")) return nullptr;
   *owner = hom::weight_colsum_insert(pb.B, pb.K, pb.N, pb.b_is_nk, *owner);
   return (*owner)->as<float>();
 }

@@ -262,3 +262,36 @@ def test_calls_on_two_streams_do_not_share_their_sums(hom, cuda):
         assert_close_f16(d[4].cpu().numpy(), case[4], "first call")
         for tD in d[5:]:
             assert torch.equal(tD, d[4])
+
+
+@pytest.mark.parametrize("declared", [False, True])
+def test_a_first_call_beside_a_capture(hom, cuda, declared):
+    """The first call for a declared weight, or on a new stream, allocates (and waits); it may do so
+    while the same thread captures another stream (torch's default capture mode), and leaves that
+    capture valid."""
+    import torch
+
+    cases = [_case(64, 256, 128, seed) for seed in (51, 52)]
+    (A, B, V, M, D), (A2, B2, V2, M2, D2) = [
+        [to_dev(x, cuda) for x in c[:4]] + [torch.zeros((1, 64, 256), dtype=torch.float16, device=cuda)]
+        for c in cases]
+    captured, beside = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    if declared:
+        hom.declare_weights(B2)
+    try:
+        with torch.cuda.graph(graph, stream=captured):
+            hom.set_stream(captured.cuda_stream)
+            hom.cutlassLayernormGemmF16(A, B, None, D, V, M)
+            hom.set_stream(beside.cuda_stream)
+            hom.cutlassLayernormGemmF16(A2, B2, None, D2, V2, M2)
+            hom.set_stream(captured.cuda_stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_close_f16(D.cpu().numpy(), cases[0][4], "captured")
+        assert_close_f16(D2.cpu().numpy(), cases[1][4], "beside the capture")
+    finally:
+        hom.use_torch_stream()
+        if declared:
+            hom.forget_weights(B2)
