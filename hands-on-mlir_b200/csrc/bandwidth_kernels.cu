@@ -529,11 +529,6 @@ inline int grid_for(long long work_items, int per_block) {
   return static_cast<int>(blocks);
 }
 
-// Dynamic shared memory the one-wave LayerNorm launches ask for and do not use: it keeps the
-// CTAs of a small GEMM (more than 180 KB each) from becoming resident beside a LayerNorm CTA that
-// they depend on, and still lets the four 16-warp CTAs an SM has threads for run at once.
-constexpr size_t kLnSmemPad = 47 * 1024;
-
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -555,7 +550,6 @@ bool layernorm_f16(const __half *x, const __half *res, const __half *gamma, cons
   })
   const unsigned blocks = static_cast<unsigned>((rows + warps_per_block - 1) / warps_per_block);
   const unsigned threads = 32u * warps_per_block;
-  const size_t smem_pad = warps_per_block == 16 ? kLnSmemPad : 0;
   const bool vec_ok = hidden % 8 == 0 && hidden <= 32 * 8 * 16 && aligned16(x) && aligned16(out) &&
                       (!res || aligned16(res)) && (!gamma || aligned16(gamma)) &&
                       (!beta || aligned16(beta));
@@ -564,7 +558,7 @@ bool layernorm_f16(const __half *x, const __half *res, const __half *gamma, cons
     const int nvec = static_cast<int>(hidden / 8);
     const int vpt = (nvec + 31) / 32;
 #define HOM_LN_CASE(V)                                                                            \
-  err = launch_pdl(layernorm_f16_warp_kernel<V, false>, dim3(blocks), dim3(threads), smem_pad, stream, 1, x, \
+  err = launch_pdl(layernorm_f16_warp_kernel<V, false>, dim3(blocks), dim3(threads), 0, stream, 1, x, \
                    res, gamma, beta, out, static_cast<long long>(rows), static_cast<int>(hidden),  \
                    eps, EmbedArgs{})
     if (vpt <= 1) HOM_LN_CASE(1);
@@ -592,7 +586,6 @@ bool embedding_layernorm_f16(const int64_t *ids, const int64_t *types, const __h
   const int warps_per_block = rows <= 8192 ? 16 : 4;
   const unsigned blocks = static_cast<unsigned>((rows + warps_per_block - 1) / warps_per_block);
   const unsigned threads = 32u * warps_per_block;
-  const size_t smem_pad = warps_per_block == 16 ? kLnSmemPad : 0;
   EmbedArgs emb;
   emb.ids = reinterpret_cast<const long long *>(ids);
   emb.types = reinterpret_cast<const long long *>(types);
@@ -605,7 +598,7 @@ bool embedding_layernorm_f16(const int64_t *ids, const int64_t *types, const __h
   const int vpt = (static_cast<int>(hidden / 8) + 31) / 32;
   cudaError_t err = cudaSuccess;
 #define HOM_EMB_CASE(V)                                                                           \
-  err = launch_pdl(layernorm_f16_warp_kernel<V, true>, dim3(blocks), dim3(threads), smem_pad, stream, 1,  \
+  err = launch_pdl(layernorm_f16_warp_kernel<V, true>, dim3(blocks), dim3(threads), 0, stream, 1,  \
                    word_emb, none, none, none, out, static_cast<long long>(rows),                  \
                    static_cast<int>(hidden), eps, emb)
   if (vpt <= 1) HOM_EMB_CASE(1);

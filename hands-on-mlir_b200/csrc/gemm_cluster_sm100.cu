@@ -34,6 +34,9 @@ constexpr int BK = 64;
 constexpr int kExchangeWarps = 8;
 constexpr int kClusterThreads = 32 * (2 + kExchangeWarps);
 constexpr uint32_t kABytes = BM * BK * 2;
+// sm_100: shared memory of an SM, what each resident CTA takes of it besides its own request, and
+// the largest request.
+constexpr uint32_t kSmSmem = 228 * 1024, kCtaReservedSmem = 1024, kMaxCtaSmem = 227 * 1024;
 // S * ceil(128 / S) rows for S = 2..8 (largest: 7 x 19)
 constexpr uint32_t kRecvRows = 136;
 
@@ -41,13 +44,17 @@ template <int BN>
 struct ClusterCfg {
   static constexpr uint32_t kBBytes = BN * BK * 2;
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  // The ring beside the receive buffer.  Both sizes stay above 180 KB on purpose: with it no CTA
-  // of a neighbouring kernel of the chain (attention 50 KB, LayerNorm 47 KB) shares an SM with
-  // this one.
-  static constexpr int kStages = BN == 64 ? 6 : 4;
+  static constexpr int kStages = BN == 64 ? 6 : 4;  // the ring, beside the receive buffer
   static constexpr uint32_t kRecvBytes = kRecvRows * BN * 4;
   static constexpr uint32_t kBarrierBytes = 8 * (2 * kStages + 1) + 16;
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + kRecvBytes + kBarrierBytes + 1024;
+  // What the kernel uses (183 / 200 KB), and what it asks for: all that a CTA can have.  Its 320
+  // threads leave half of an SM's registers and threads free, and no CTA of this kernel may sit
+  // beside a CTA of the previous kernel that it depends on (or of the next one): with all of the
+  // shared memory taken nothing else fits, whatever the other kernel needs.
+  static constexpr uint32_t kUsedBytes = kStages * kStageBytes + kRecvBytes + kBarrierBytes + 1024;
+  static constexpr uint32_t kSmemBytes = kMaxCtaSmem;
+  static_assert(kUsedBytes <= kSmemBytes, "ring and receive buffer exceed a CTA's shared memory");
+  static_assert(kSmemBytes + 2 * kCtaReservedSmem > kSmSmem, "another CTA would fit beside this one");
 };
 
 struct ClusterParams {
