@@ -381,6 +381,20 @@ bool cluster_supported(const Problem &pb, int parts) {
          !has_layernorm_form(pb);
 }
 
+// A split that a caller or a tuned entry asks for may have many more tiles than clusters run at
+// once.  Every further wave of clusters is a kernel start of its own, while the serial form runs on
+// persistent CTAs; its parts of a tile wait for one another, though, which is only short when they
+// run in the same round, that is when the number of SMs is a multiple of the factor (2 and 4 of
+// 148).  Measured, serial against cluster form in us: with 2 parts 128 tiles (2048 x 1024 x 1024,
+// 128 wide) 15.3 / 15.5, 192 tiles (4096 x 768 x 3072, 128 wide) 27.9 / 36.7, 768 tiles
+// (4096 x 3072 x 768, 128 wide) 54 / 81; with 4 parts 128 tiles 33.6 / 31.6, 192 tiles 50 / 61, 768
+// tiles 117 / 181; but with 3 parts 768 tiles 156 / 130, with 8 parts 714 / 381.  So the line for 2
+// and 4 is where the tiles alone fill the chip once.
+bool cluster_pays(const Problem &pb, int bn, int parts) {
+  const int64_t tiles = ((pb.M + BM - 1) / BM) * ((pb.N + bn - 1) / bn);
+  return sm_count() % parts != 0 || tiles <= parts * cluster_capacity(bn, parts);
+}
+
 int cluster_capacity(int bn, int parts) {
   // Clusters of more than two CTAs need SMs of one GPC; how many fit depends on which SMs of each
   // GPC the device has.  Asked once per device; the fallback is a 148-SM part (and what a build

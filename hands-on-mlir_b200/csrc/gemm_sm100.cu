@@ -1302,10 +1302,12 @@ bool run(const Problem &pb, int tile_row, cudaStream_t stream) {
       return false;
     }
   }
+  split = clamp_split(split, static_cast<int>((pb.K + BK - 1) / BK));
   const TileRow &t = kTileRows[tile_row];
   if (t.pair) return run_pair(pb, t.tile_n, split, stream);
   // 128 x {64,128} tiles with a short K split: one cluster per tile, parts reduced SM to SM.
-  if (tile_row <= 2 && cluster_supported(pb, split)) return run_cluster(pb, t.tile_n, split, stream);
+  if (tile_row <= 2 && cluster_supported(pb, split) && cluster_pays(pb, t.tile_n, split))
+    return run_cluster(pb, t.tile_n, split, stream);
   if (pb.b_is_nk) {
     switch (t.tile_n) {
       case 64: return launch_variant<64, true>(pb, split, stream);

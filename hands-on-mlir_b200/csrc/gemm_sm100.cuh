@@ -75,9 +75,11 @@ bool layernorm_fusion_shape(int64_t n, int *cluster_n, int *bn);
 bool run_pair(const Problem &pb, int bn2, int split_k, cudaStream_t stream);
 
 // One cluster of `parts` CTAs per 128 x {64,128} tile, K split over the cluster
-// (gemm_cluster_sm100.cu); cluster_supported says whether `pb` can run on it.
+// (gemm_cluster_sm100.cu); cluster_supported says whether `pb` can run on it, cluster_pays whether
+// it is faster there than as a serial split.
 constexpr int kMaxClusterParts = 8;
 bool cluster_supported(const Problem &pb, int parts);
+bool cluster_pays(const Problem &pb, int bn, int parts);
 bool run_cluster(const Problem &pb, int bn, int parts, cudaStream_t stream);
 // How many clusters of `parts` CTAs the device runs at once (128 x bn tiles).
 int cluster_capacity(int bn, int parts);

@@ -53,6 +53,20 @@ def test_cluster_split_matches_the_oracle(hom, cuda, oracle, row, m, n, k, split
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("row,m,n,k,split", [
+    (1, 1024, 1152, 256, 2),  # 144 tiles: clusters, the second wave partly filled
+    (1, 1024, 1208, 256, 2),  # 152 tiles: serial split on persistent CTAs
+    (2, 1281, 1400, 264, 4),  # 121 tiles, clusters
+    (2, 1409, 1480, 264, 4),  # 144 tiles, serial
+    (1, 300, 200, 136, 16),   # more parts than K blocks: three, as clusters
+])
+def test_asked_for_splits_on_both_sides_of_the_rule(hom, cuda, oracle, row, m, n, k, split):
+    A, B, C = _operands(m, n, k, 3000 + m + split)
+    got = _run(hom, cuda, A, B, C, row=row, split=split, beta=1.0)
+    assert_close_f16(got, oracle.gemm_f16(A, B, C, beta=1.0), "residual")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(16, 768, 768), (64, 2304, 768), (77, 768, 3072), (200, 1024, 4096)])
 def test_automatic_choice_with_weights_stored_nk(hom, cuda, oracle, m, n, k):
     assert hom.gemm_query_tile(m, n, k, 0)["split_k"] >= 2
