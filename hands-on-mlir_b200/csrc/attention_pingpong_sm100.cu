@@ -42,6 +42,7 @@
 // Same contract as the reference's cuDNN fused attention behind TransformerEngine
 // (include/NVGPUKernels/BertAttentionRunner.h:52-136: layout BS3HD, no bias, padding mask,
 // no dropout, inference).
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 
@@ -76,11 +77,13 @@ constexpr uint32_t kTmemColsPP = 512;
 
 constexpr float kLazyGrowth = 8.0f;
 
-// Registers per thread after the hand-over between the warpgroups.  A thread of the launch has
-// 65,536 / 384 rounded down to a multiple of 8; the shares must not add up to more than three of
-// those (run_pingpong checks the compiled count), or the increase would wait for good.
-constexpr int kLaunchRegs = 168, kControlRegs = 72, kSoftmaxRegs = 216;
-static_assert(kControlRegs + 2 * kSoftmaxRegs <= 3 * kLaunchRegs, "register shares exceed the launch's");
+// Registers per thread after the hand-over between the warpgroups.  The shares of the three must not
+// add up to more than what the launch gave them, or the increase would wait for good.  How many a
+// thread of the launch has is the compiler's choice, at most 65,536 / 384 rounded down to a multiple
+// of 8 (168), so pingpong_available() looks at the compiled count before the kernel is ever run.
+constexpr int kControlRegs = 72, kSoftmaxRegs = 216;
+constexpr bool hand_over_fits(int launch_regs) { return kControlRegs + 2 * kSoftmaxRegs <= 3 * launch_regs; }
+static_assert(hand_over_fits(168) && !hand_over_fits(160), "the shares use all that a launch can have");
 
 struct ParamsPP {
   const int *cu_seqlens;
@@ -593,6 +596,22 @@ attention_f16_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const _
 
 }  // namespace
 
+bool pingpong_available() {
+  static std::atomic<int> launch_regs[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  int regs = launch_regs[dev].load(std::memory_order_relaxed);
+  if (regs == 0) {
+    cudaFuncAttributes fa;
+    if (!check_cuda(cudaFuncGetAttributes(&fa, attention_f16_pingpong_kernel), "cudaFuncGetAttributes(attention)"))
+      return false;
+    regs = fa.numRegs;
+    launch_regs[dev].store(regs, std::memory_order_relaxed);
+  }
+  return hand_over_fits(regs);
+}
+
 bool run_pingpong(const Problem &pb, cudaStream_t stream) {
   static bool attr_set[64] = {};
   int dev = 0;
@@ -602,14 +621,6 @@ bool run_pingpong(const Problem &pb, cudaStream_t stream) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesPP),
                     "cudaFuncSetAttribute(attention, two query tiles per CTA)"))
       return false;
-    cudaFuncAttributes fa;
-    if (!check_cuda(cudaFuncGetAttributes(&fa, attention_f16_pingpong_kernel), "cudaFuncGetAttributes(attention)"))
-      return false;
-    if (fa.numRegs < kLaunchRegs) {  // see kLaunchRegs
-      set_error(HOM_ERR_UNSUPPORTED, "attention: the kernel was built with %d registers, its hand-over needs %d",
-                fa.numRegs, kLaunchRegs);
-      return false;
-    }
     attr_set[dev] = true;
   }
   CUtensorMap tm;

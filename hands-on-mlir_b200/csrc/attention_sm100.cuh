@@ -21,6 +21,8 @@ bool run(const Problem &pb, cudaStream_t stream);
 bool make_out_map(const void *ptr, uint64_t hidden, uint64_t seq, uint64_t bs, uint32_t box_rows, CUtensorMap *out);
 // seq > 128: the persistent kernel that owns two query tiles per CTA (attention_pingpong_sm100.cu).
 bool run_pingpong(const Problem &pb, cudaStream_t stream);
+// False when this build of it cannot hand its registers over; the general kernel serves the call then.
+bool pingpong_available();
 
 }  // namespace attention
 }  // namespace hom
