@@ -75,6 +75,40 @@ def test_automatic_choice_with_weights_stored_nk(hom, cuda, oracle, m, n, k):
     assert_close_f16(got, oracle.gemm_f16(A, B, C, beta=1.0), "[1, N, K] weights")
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("nk", [False, True])
+@pytest.mark.parametrize("m,n,k,split", [(64, 1024, 4096, 8), (200, 136, 3072, 2), (128, 768, 3072, 5)])
+def test_declared_weights_with_a_share_longer_than_the_ring(hom, cuda, oracle, m, n, k, split, nk, tmp_path):
+    """The first K blocks of a declared weight are requested before the kernel that writes A has
+    finished, the others as the ring (six stages, four with 128 columns) comes round."""
+    import torch
+
+    A, B, C = _operands(m, n, k, 4000 + m)
+    want = oracle.gemm_f16(A, B, C, beta=1.0)
+    tB = to_dev(np.ascontiguousarray(B.transpose(0, 2, 1)) if nk else B, cuda)
+    half, tC = to_dev(A / 2, cuda), to_dev(C, cuda)
+    tA = torch.zeros((1, m, k), dtype=torch.float16, device=cuda)
+    tD = torch.zeros((1, m, n), dtype=torch.float16, device=cuda)
+    table = tmp_path / "tuned.txt"
+    hom.declare_weights(tB)
+    try:
+        for row, stages in ((1, 6), (2, 4)):
+            assert -(-k // 64) // split > stages
+            table.write_text(f"{m} {n} {k} 0 {row} {split}\n")  # the [N, K] entry takes its split from here
+            assert hom.gemm_tune_load(table) == 1
+            for _ in range(3):
+                tA.zero_()
+                hom.elementwise("Add", "F16", half, half, tA)
+                if nk:
+                    hom.nvteGemmF16(tA, tB, tC, tD, beta=1.0)
+                else:
+                    hom.cutlassGemmF16(tA, tB, tC, tD, beta=1.0)
+                hom.synchronize()
+                assert_close_f16(tD.cpu().numpy(), want, f"row {row}")
+    finally:
+        hom.forget_weights(tB)
+
+
 def test_the_rule_splits_only_where_all_clusters_run_at_once(hom):
     """Rows 1 and 2, at most eight parts, no more parts than K blocks, no more CTAs than SMs; no
     split at all where N is not a multiple of 8 or the output has more tiles than the chip."""
