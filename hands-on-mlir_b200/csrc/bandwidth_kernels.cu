@@ -287,7 +287,8 @@ repitch_rows_f16_kernel(const __half *src, __half *dst, long long rows, int cols
 // contiguous bytes per warp and load, eight loads in flight), then the 32 partial sums of a column
 // are added in warp order.  Bound by latency: one thread per column walking all K rows took 46 us
 // at 768 x 3072, this form 3 us.
-// [N, K]: one warp per row of b, 16-byte loads where rows are aligned.
+// [N, K]: one warp per row of b, 16-byte loads.
+// b is 16-byte aligned, K and N are multiples of 8 (what the entry points accept).
 constexpr int kColSumWarps = 32;
 
 __global__ void __launch_bounds__(32 * kColSumWarps)
@@ -300,20 +301,16 @@ col_sum_f16_kernel(const __half *b, float *out, int k_dim, int n_dim, int b_is_n
     if (n >= n_dim) return;
     const __half *row = b + static_cast<long long>(n) * k_dim;
     float s = 0.f;
-    if ((k_dim & 7) == 0 && (reinterpret_cast<uintptr_t>(b) & 15u) == 0) {
-      const uint4 *v = reinterpret_cast<const uint4 *>(row);
+    const uint4 *v = reinterpret_cast<const uint4 *>(row);
 #pragma unroll 4
-      for (int i = lane; i < (k_dim >> 3); i += 32) {
-        const uint4 raw = v[i];
-        const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
+    for (int i = lane; i < (k_dim >> 3); i += 32) {
+      const uint4 raw = v[i];
+      const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(h2[j]);
-          s += f.x + f.y;
-        }
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(h2[j]);
+        s += f.x + f.y;
       }
-    } else {
-      for (int k = lane; k < k_dim; k += 32) s += __half2float(row[k]);
     }
     s = warp_sum(s);
     if (lane == 0) out[n] = s;
@@ -322,20 +319,12 @@ col_sum_f16_kernel(const __half *b, float *out, int k_dim, int n_dim, int b_is_n
   __shared__ float2 part[kColSumWarps][32];
   const int n = blockIdx.x * 64 + 2 * lane;
   float2 s = make_float2(0.f, 0.f);
-  if ((n_dim & 1) == 0 && (reinterpret_cast<uintptr_t>(b) & 3u) == 0) {  // pairs are 4-byte aligned
-    if (n < n_dim) {
+  if (n < n_dim) {
 #pragma unroll 8
-      for (int k = warp; k < k_dim; k += kColSumWarps) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(b + static_cast<long long>(k) * n_dim + n));
-        s.x += f.x;
-        s.y += f.y;
-      }
-    }
-  } else {
     for (int k = warp; k < k_dim; k += kColSumWarps) {
-      const __half *p = b + static_cast<long long>(k) * n_dim + n;
-      if (n < n_dim) s.x += __half2float(p[0]);
-      if (n + 1 < n_dim) s.y += __half2float(p[1]);
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(b + static_cast<long long>(k) * n_dim + n));
+      s.x += f.x;
+      s.y += f.y;
     }
   }
   part[warp][lane] = s;

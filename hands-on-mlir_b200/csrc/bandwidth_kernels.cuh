@@ -37,7 +37,8 @@ bool row_stats_finalize(const float2 *partials, int groups, int64_t rows, int64_
                         __half *shift_out, cudaStream_t stream);
 bool row_stats_f16(const __half *x, __half *rstd_out, __half *shift_out, int64_t rows, int64_t n,
                    float eps, cudaStream_t stream);
-// out[n] = sum over k of B[k, n] (or B[n, k] when b_is_nk), fp32.
+// out[n] = sum over k of B[k, n] (or B[n, k] when b_is_nk), fp32; B 16-byte aligned, K and N
+// multiples of 8.
 bool col_sum_f16(const __half *b, float *out, int64_t k_dim, int64_t n_dim, bool b_is_nk,
                  cudaStream_t stream);
 

@@ -5,8 +5,9 @@
 // 100 output tiles, and what a launch costs is the chain one CTA goes through: the 64-deep K
 // blocks of its tile one after the other, as fast as a single SM can pull them (a 128 x 64 tile
 // of K = 3072 is 1.2 MB), on a chip that is mostly idle.  Here S = 2..8 CTAs share a tile, each
-// accumulates its K blocks in its own tensor memory (all of its operand tiles fit the ring, so
-// they are requested at once, the weights even before the previous kernel has finished), and the
+// accumulates its K blocks in its own tensor memory (the first six, with 128-column tiles four, are
+// requested at once, their weights even before the previous kernel has finished; a longer share
+// goes round the ring), and the
 // partial tiles are exchanged SM to SM: CTA r of the cluster owns rows [r, r + 1) * ceil(rows / S)
 // of the tile, every CTA stores the rows of its partial accumulator straight into their owner's
 // shared memory, and after one cluster barrier the owner adds the S parts in part order (the sum

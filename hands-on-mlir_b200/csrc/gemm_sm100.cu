@@ -15,8 +15,8 @@
 //               tile are reduced serially through an fp32 workspace (SplitK, gemm_epilogue.cuh).
 //
 // This replaces the reference's CUTLASS 2.x mma.sync kernels and its compile-time autotuner
-// (include/NVGPUKernels/GemmRunner.h:119-310, lib/NVGPUKernels/GemmProfiler.cu:143-236) with a
-// small per-shape tile table.
+// (include/NVGPUKernels/GemmRunner.h:119-310, lib/NVGPUKernels/GemmProfiler.cu:143-236) with six
+// tile shapes, an estimate of their times that picks one, and a tuner whose choices come first.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -974,11 +974,6 @@ bool tuned_choice(int64_t m, int64_t n, int64_t k, int act, int *row, int *split
   if (row) *row = it->second.row;
   if (split) *split = it->second.split;
   return true;
-}
-
-int tuned_row(int64_t m, int64_t n, int64_t k, int act) {
-  int row = 0;
-  return tuned_choice(m, n, k, act, &row, nullptr) ? row : 0;
 }
 
 // Text lines "M N K activation row [split]" (split defaults to 1).

@@ -26,7 +26,7 @@ struct Problem {
   float alpha = 1.f, beta = 0.f;
   int act = 0;  // 1 = erf GELU
   // K parts per output tile: >= 2 as given (clamped to the number of 64-wide K blocks and 16),
-  // anything else lets the tile table / tuner / heuristic decide.
+  // anything else leaves it to a tuned entry or the cost estimate.
   int split_k = 0;
   // LayerNorm-on-A form (all null when unused): D = epilogue(alpha * (A * row_scale + row_shift).B ...)
   // evaluated as row_scale[r] * (A.B)[r,n] + row_shift[r] * col_sum[n] with col_sum = column sums of B.
@@ -62,7 +62,7 @@ inline int epilogue_kind(const Problem &pb) {
 }
 
 // Enqueues the GEMM; tile_row 1..4 forces one CTA per 128 x {64,128,192,256} tile, 5..6 one
-// CTA pair per 256 x {128,256} tile; anything else lets the tile table / heuristic decide.
+// CTA pair per 256 x {128,256} tile; anything else leaves it to a tuned entry or the estimate.
 // Returns false (error recorded) on failure.
 bool run(const Problem &pb, int tile_row, cudaStream_t stream);
 // D = LayerNorm(fp16(A.B + C)) over the last dimension, no affine (C: c_mode 0 or 1; alpha, beta,
@@ -97,7 +97,6 @@ int query_tile(int64_t m, int64_t n, int64_t k, int act, int *bn, int *stages, i
 // the winner for later automatic selections, and can persist the table as text.
 bool tune(int64_t m, int64_t n, int64_t k, int act, float alpha, float beta, bool b_is_nk, int iters,
           int *best_row, int *best_split, float *best_us, float *row_us, cudaStream_t stream);
-int tuned_row(int64_t m, int64_t n, int64_t k, int act);
 bool tuned_choice(int64_t m, int64_t n, int64_t k, int act, int *row, int *split);
 int tune_cache_load(const char *path);  // entries read, or -1
 int tune_cache_save(const char *path);  // entries written, or -1

@@ -27,16 +27,16 @@ enum DeviceError : int {
   kDevWaitTimeoutMma = 102,
   kDevWaitTimeoutEpilogue = 103,
   kDevWaitTimeoutAttention = 104,
-  kDevWaitTimeoutDrain = 105,
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// One lane of the (converged) warp gets true.  Code that is executed by the whole warp with
-// only the asynchronous instruction itself under this predicate keeps its address and
-// descriptor arithmetic warp-uniform, which is what lets it run on the uniform datapath.
+// One lane of the (converged) warp gets true, the same one every time.  A producer or issuer puts
+// its whole loop under one election: the compiler then knows that a single thread runs it, while an
+// election per instruction costs votes and reconvergence around each (the measurements stand at the
+// MMA issuer of gemm_sm100.cu).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -134,21 +134,6 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
       "}\n"
       : "=r"(done)
       : "r"(bar), "r"(parity), "r"(ns)
-      : "memory");
-  return done != 0;
-}
-
-// Non-blocking probe of a phase.
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred P;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, P;\n\t"
-      "}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
       : "memory");
   return done != 0;
 }
