@@ -47,9 +47,6 @@ struct EpilogueParams {
   // finalising kernel turns them into 1/sqrt(var + eps) and -mean/sqrt(var + eps).  This is what
   // the reference's epilogue visitor does per N-tile (include/NVGPUKernels/Layernorm.h:409-479).
   float2 *row_partials;
-  // Diagnostics builds: bit mask that removes parts of the epilogue (1 accumulator read,
-  // 2 arithmetic, 4 staging stores, 8 global store, 16 C read, 32 everything but the release).
-  HOM_DIAG(int dbg;)
 };
 
 // GELU on two values at once for the tile epilogues, built so that the special-function unit
@@ -157,7 +154,7 @@ __device__ __forceinline__ void row_stats_from_partials(const float2 *partials, 
 // Called before the accumulator wait so that the loads hide behind the main loop.
 __device__ __forceinline__ RowAffine epilogue_row_affine(const EpilogueParams &ep, int row) {
   RowAffine ra;
-  if (row >= ep.M HOM_DIAG(|| (ep.dbg & 2048))) return ra;
+  if (row >= ep.M) return ra;
   if (ep.row_scale != nullptr) {
     ra.rs = __half2float(ep.row_scale[row]);
     ra.sh = __half2float(ep.row_shift[row]);
@@ -176,7 +173,7 @@ __device__ __forceinline__ RowAffine epilogue_row_affine(const EpilogueParams &e
 // round trip would be in the open.
 __device__ __forceinline__ float2 epilogue_load_col_sums(const EpilogueParams &ep, int c0, int lane) {
   float2 cs = make_float2(0.f, 0.f);
-  if (ep.col_sum == nullptr HOM_DIAG(|| (ep.dbg & 4096))) return cs;
+  if (ep.col_sum == nullptr) return cs;
   // (L2 loads: both these sums, when B is not a declared weight, and the row statistics above
   // were written by the kernel just before this one)
   if (c0 + lane < ep.N) cs.x = __ldcg(ep.col_sum + c0 + lane);
@@ -189,10 +186,6 @@ __device__ __forceinline__ float2 epilogue_load_col_sums(const EpilogueParams &e
 template <int G0 = 0, int G1 = 8, bool ALIGNED_ONLY = false>
 __device__ __forceinline__ void epilogue_load_c(const EpilogueParams &ep, int row, int c0, uint4 (&cval)[8]) {
   if (ep.c_mode == 0) return;
-  HOM_DIAG(if (ep.dbg & 48) {
-    for (int g = G0; g < G1; ++g) cval[g] = make_uint4(0, 0, 0, 0);
-    return;
-  })
   const __half *cp = ep.c_mode == 1 ? ep.C + static_cast<long long>(row) * ep.ldc + c0 : ep.C + c0;
   const bool row_ok = ep.c_mode == 2 || row < ep.M;
   if (!ALIGNED_ONLY && ep.unaligned_n) {
@@ -245,7 +238,7 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
                                                     const RowAffine ra = RowAffine(),
                                                     const float2 col_sums = float2{0.f, 0.f}) {
   using namespace hom::ptx;
-  if (!active HOM_DIAG(|| (ep.dbg & 32))) {
+  if (!active) {
     tc_fence_before_sync();
     __syncwarp();
     release();
@@ -257,7 +250,7 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
       // Wait until the parts before this one are in the slot.  One lane polls (with an acquire
       // load); the warp barrier that follows orders the other lanes' slot reads after it.
       bool ok = true;
-      if (lane == 0 HOM_DIAG(&& !(ep.dbg & 64))) {
+      if (lane == 0) {
         const long long t0 = clock64();
         for (uint32_t it = 0;; ++it) {
           int have;
@@ -315,7 +308,6 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
           __stcg(reinterpret_cast<uint4 *>(slot + (half * 8 + j) * 128),
                  make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
       }
-      HOM_DIAG(if (!(ep.dbg & 128)))
       __threadfence();
       __syncwarp();
       if (lane == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(sk.counter), "r"(sk.part + 1) : "memory");
@@ -344,16 +336,8 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
   // overlaps the first half's arithmetic).
   auto do_half = [&](const int half) {
     uint32_t acc[32];
-#if HOM_DIAG_ENABLED
-    if (ep.dbg & 1) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) acc[i] = 0x3f000000u + lane;
-    } else
-#endif
-    {
-      tmem_ld_32x32(tmem_addr + half * 32, acc);
-      tmem_ld_wait();
-    }
+    tmem_ld_32x32(tmem_addr + half * 32, acc);
+    tmem_ld_wait();
     if constexpr (SPLIT) {
       // acc <- (p0 + ... + p_{last-1}) + p_last, the left operand being what the slot holds.
       // The residual / bias values of this half are requested together with the slot (the
@@ -382,7 +366,7 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
       __syncwarp();
     }
     if constexpr (kLnA) {
-      if (ln_on_a HOM_DIAG(&& !(ep.dbg & 1024))) {
+      if (ln_on_a) {
         // acc <- rstd * acc - mean * rstd * col_sum[column]; the shuffles are warp-uniform
         const float mine = half == 0 ? col_sums.x : col_sums.y;
 #pragma unroll
@@ -406,23 +390,20 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
       for (int j = 0; j < 4; ++j) {
         const int i0 = g * 8 + 2 * j;
         float2 v = make_float2(__uint_as_float(acc[i0]), __uint_as_float(acc[i0 + 1]));
-        HOM_DIAG(if (!(ep.dbg & 2))) {
-          if constexpr (EPI == kEpiGeneric) {
-            if (!unit_alpha) v = __fmul2_rn(alpha2, v);  // alpha * x is exact for alpha == 1: skip it
-          }
-          if (EPI == kEpiAddC || (EPI == kEpiGeneric && ep.c_mode != 0)) {
-            float2 c = __half22float2(h2[j]);
-            if constexpr (kLnR) {
-              if (ln_on_r) c = __ffma2_rn(rr2, c, rt_g);
-            }
-            v = EPI == kEpiAddC ? __fadd2_rn(c, v) : __ffma2_rn(beta2, c, v);
-          }
-          if (EPI == kEpiGelu || (EPI == kEpiGeneric && ep.act == 1)) v = gelu_erf_fast2(v);
+        if constexpr (EPI == kEpiGeneric) {
+          if (!unit_alpha) v = __fmul2_rn(alpha2, v);  // alpha * x is exact for alpha == 1: skip it
         }
+        if (EPI == kEpiAddC || (EPI == kEpiGeneric && ep.c_mode != 0)) {
+          float2 c = __half22float2(h2[j]);
+          if constexpr (kLnR) {
+            if (ln_on_r) c = __ffma2_rn(rr2, c, rt_g);
+          }
+          v = EPI == kEpiAddC ? __fadd2_rn(c, v) : __ffma2_rn(beta2, c, v);
+        }
+        if (EPI == kEpiGelu || (EPI == kEpiGeneric && ep.act == 1)) v = gelu_erf_fast2(v);
         const __half2 h = __floats2half2_rn(v.x, v.y);
         w[j] = *reinterpret_cast<const uint32_t *>(&h);
         if constexpr (kStats) {
-          HOM_DIAG(if (ep.dbg & 256) continue;)
           // statistics of what is stored: the rounded values (columns beyond N hold zeros)
           const float2 q = __half22float2(h);
           s1 += q.x + q.y;
@@ -430,12 +411,6 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
         }
       }
       const uint32_t addr = my_row + ((static_cast<uint32_t>(half * 4 + g) ^ (lane & 7u)) << 4);
-#if HOM_DIAG_ENABLED
-      if (ep.dbg & 4) {
-        asm volatile("" ::"r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]));
-        continue;
-      }
-#endif
       asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]),
                    "r"(w[2]), "r"(w[3])
                    : "memory");
@@ -444,7 +419,7 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
   do_half(0);
   do_half(1);
   if constexpr (kStats) {
-    if (ep.row_partials != nullptr && row < ep.M HOM_DIAG(&& !(ep.dbg & 512)))
+    if (ep.row_partials != nullptr && row < ep.M)
       ep.row_partials[static_cast<long long>(c0 >> 6) * ep.M + row] = make_float2(s1, s2);
   }
   // (the specialised epilogues and the LayerNorm forms are only chosen when N % 8 == 0)
@@ -452,7 +427,7 @@ __device__ __forceinline__ bool epilogue_warp_block(const EpilogueParams &ep, co
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      if (c0 < ep.N && row0 < ep.M HOM_DIAG(&& !(ep.dbg & 8))) tma_store_2d(tmD, stage_smem, c0, row0);
+      if (c0 < ep.N && row0 < ep.M) tma_store_2d(tmD, stage_smem, c0, row0);
       bulk_commit_group();
     }
   } else {

@@ -693,7 +693,6 @@ bool launch_variant(const Problem &pb, int split_k, cudaStream_t stream) {
   p.ep.ln_eps = pb.ln_eps;
   p.ep.unaligned_n = pb.N % 8 != 0 ? 1 : 0;
   p.ep.row_partials = pb.row_partials;
-  HOM_DIAG(p.ep.dbg = std::getenv("HOM_EPI_DBG") ? std::atoi(std::getenv("HOM_EPI_DBG")) : 0;)
   const int m_blocks = static_cast<int>((pb.M + BM - 1) / BM);
   p.n_blocks = static_cast<int>((pb.N + BN - 1) / BN);
   p.num_tiles = m_blocks * p.n_blocks;
@@ -772,7 +771,6 @@ bool launch_ln_variant(const Problem &pb, float eps, cudaStream_t stream) {
   p.ep.a_inv_n = p.ep.r_inv_n = p.ep.ln_eps = 0.f;
   p.ep.unaligned_n = 0;
   p.ep.row_partials = nullptr;
-  HOM_DIAG(p.ep.dbg = 0;)
   const int m_blocks = static_cast<int>((pb.M + BM - 1) / BM);
   p.n_blocks = static_cast<int>(pb.N / BN);
   p.num_tiles = m_blocks * p.n_blocks;
@@ -901,7 +899,6 @@ bool run_fixed_no_alloc(const Problem &pb, cudaStream_t stream) {
   p.ep.ln_eps = pb.ln_eps;
   p.ep.unaligned_n = pb.N % 8 != 0 ? 1 : 0;
   p.ep.row_partials = pb.row_partials;
-  HOM_DIAG(p.ep.dbg = std::getenv("HOM_EPI_DBG") ? std::atoi(std::getenv("HOM_EPI_DBG")) : 0;)
   p.b_grouped = grouped ? 1 : 0;
   p.b_early = pb.b_const ? 1 : 0;
   const int m_blocks = static_cast<int>((pb.M + BM - 1) / BM);
