@@ -20,6 +20,8 @@
 // to a reference that only follows the row's running maximum when that has grown by more than
 // 2^8 (kLazyGrowth): until then P is at most 256 (fp16 keeps its relative precision there, the
 // row sum is fp32), and the threads neither rescale O nor wait for the product before.
+// (Two query tiles per CTA, the lazily followed maximum and P as a tensor-memory operand are steps
+// of the published FlashAttention-4 algorithm.)
 //
 // What bounds it: the exponentials.  ex2 runs on the special-function unit at 16 per clock and
 // SM, 2,048 clk for one KV step of both tiles.  (Evaluating one, two or three pairs of eight by a

@@ -189,10 +189,13 @@ HOM_EXPORT int homSynchronize(void);
  * returned by allocConstantNVGPU* are declared by the library; callers that bring their own
  * weight buffers may declare them to get the earlier prefetch.  homForgetWeights() withdraws a
  * declaration (call it before the buffer is freed or reused).  What the library derives from a
- * declared weight and keeps (a re-pitched copy for N % 8 != 0, column sums for the deferred
- * LayerNorm) is dropped when the weight is forgotten and when it is declared again: declare a
- * buffer again after rewriting its contents.  No counterpart in the reference, whose launches
- * are fully serialised on the null stream. */
+ * declared weight and keeps (a re-pitched copy for N % 8 != 0; column sums for
+ * cutlassLayernormGemmF16 and the deferred LayerNorm) is dropped when the weight is forgotten and
+ * when it is declared again: declare a buffer again after rewriting its contents.  The first call
+ * that derives something allocates and waits for its stream.  A captured cutlassLayernormGemmF16
+ * computes its sums inside the graph; a graph captured with one of the other kept buffers shares
+ * their ownership, so it stays valid, but has to be captured again to follow a new declaration.
+ * No counterpart in the reference, whose launches are fully serialised on the null stream. */
 HOM_EXPORT void homDeclareWeights(const void *ptr, int64_t bytes);
 HOM_EXPORT void homForgetWeights(const void *ptr);
 
@@ -245,9 +248,9 @@ HOM_EXPORT void homBertEmbeddingF16(int64_t rankIds, void *dstIds, int64_t rankT
  * express BERT's normalised residual.  A [.., M, K], B [1, K, N] or [1, N, K] (weightsNK),
  * R, D [.., M, N], N % 8 == 0; activation 0 or 1 (erf GELU).  StatsD must not be the buffer
  * of StatsA or StatsR (other tiles still read them).  With StatsA, the first call for a declared
- * weight computes and caches its column sums (allocates device memory and waits for the stream):
- * make that call outside of any stream capture; for any other B the sums are recomputed by an
- * extra launch on every call (N <= 65536). */
+ * weight computes and caches its column sums (allocates device memory and waits for the stream).
+ * For any other B, and for a declared weight that is first seen under stream capture, an extra
+ * launch recomputes them on every call or replay (N <= 65536). */
 HOM_EXPORT void homGemmDeferredLayernormF16(int64_t rankA, void *dstA, int64_t rankStatsA, void *dstStatsA,
                                             int64_t rankB, void *dstB, bool weightsNK, int64_t rankR,
                                             void *dstR, int64_t rankStatsR, void *dstStatsR, int64_t rankD,
