@@ -170,6 +170,8 @@ void free_released_memory() {
     std::lock_guard<std::mutex> lock(list.mu);
     ptrs.swap(list.ptrs);
   }
+  if (ptrs.empty()) return;
+  CaptureSafeCalls safe;
   for (void *ptr : ptrs) cudaFree(ptr);
 }
 }  // namespace
@@ -181,8 +183,8 @@ DeviceBuffer::~DeviceBuffer() {
 }
 
 SharedBuffer device_buffer(size_t bytes, const char *what) {
-  CaptureSafeCalls safe;
   free_released_memory();
+  CaptureSafeCalls safe;
   void *ptr = nullptr;
   if (!check_cuda(cudaMalloc(&ptr, bytes), what)) return nullptr;
   return std::make_shared<DeviceBuffer>(ptr);

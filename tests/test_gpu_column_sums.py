@@ -143,10 +143,12 @@ def test_a_captured_call_follows_a_rewritten_weight(hom, cuda):
 
 def test_captured_calls_do_not_share_their_sums(hom, cuda):
     """Two graphs captured on one stream, with different weights, replayed on two streams at once;
-    then both destroyed and captured again."""
+    then both destroyed and captured again, their memory being given back in the meantime (by the
+    declaration inside the next capture, or before)."""
     import torch
 
     cases = [_case(256, 512, 512, seed) for seed in (21, 22)]
+    other = torch.zeros(64, dtype=torch.float16, device=cuda)
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
     dev = [[to_dev(x, cuda) for x in c[:4]] + [torch.zeros((1, 256, 512), dtype=torch.float16, device=cuda)]
            for c in cases]
@@ -157,6 +159,8 @@ def test_captured_calls_do_not_share_their_sums(hom, cuda):
             graphs = [torch.cuda.CUDAGraph() for _ in cases]
             for graph, (tA, tB, tV, tM, tD) in zip(graphs, dev):
                 with torch.cuda.graph(graph, stream=streams[0]):
+                    hom.declare_weights(other)
+                    hom.forget_weights(other)
                     for _ in range(8):
                         hom.cutlassLayernormGemmF16(tA, tB, None, tD, tV, tM)
             for _ in range(20):
@@ -167,7 +171,8 @@ def test_captured_calls_do_not_share_their_sums(hom, cuda):
             for case, d in zip(cases, dev):
                 assert_close_f16(d[4].cpu().numpy(), case[4], "replayed on two streams")
                 d[4].zero_()
-            del graphs
+            del graph, graphs
+            time.sleep(0.2)  # CUDA reports the end of a graph from a thread of its own
     finally:
         hom.use_torch_stream()
 
